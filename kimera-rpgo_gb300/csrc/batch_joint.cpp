@@ -421,6 +421,7 @@ int solve_joint(int dim, std::vector<JointProblem*>& probs, cudaStream_t st, int
       }
       if (!(c & kBatchActive)) continue;
       const double errx = res[g], nerr = res[G + g], lin_change = res[2 * G + 2 * g];
+      chol_check_status(res[2 * G + 2 * g + 1]);
       const bool ok = res[2 * G + 2 * g + 1] == 0.0;
       if (x.phase == Graph::kLmStart) {
         x.cur_err = errx;

@@ -222,8 +222,7 @@ void multirobot_align(rpgo_solver* s) {
     }
     const uint64_t key0 = 0;
     vs.append(1, &key0, ident.data(), false, s->st);
-    GpuNls nls(s->dim, graph, fs, vs, s->st, true);
-    nls.dev().coop_ctas = s->coop_ctas;
+    GpuNls nls(s->dim, graph, fs, vs, s->st, true, s->coop_ctas);
     GncConfig g;
     if (s->p.multirobot_align_method == RPGO_ALIGN_L2) {
       g.threshold_mode = RPGO_GNC_COST;
@@ -300,8 +299,7 @@ int optimize(rpgo_solver* s) {
       init.assign(full.size(), 0.0);
       for (size_t i = 0; i < n_known && i < init.size(); ++i) init[i] = 1.0;
     }
-    GpuNls nls(s->dim, full, *s->store, sv.get(), s->st, s->p.linear_solver != RPGO_LINEAR_PCG);
-    nls.dev().coop_ctas = s->coop_ctas;
+    GpuNls nls(s->dim, full, *s->store, sv.get(), s->st, s->p.linear_solver != RPGO_LINEAR_PCG, s->coop_ctas);
     const int wm = s->p.gnc_warm_start;
     if (wm == RPGO_WARM_ON || wm == RPGO_WARM_RECORD || wm == RPGO_WARM_CONTINUATION)
       closure_features_and_probs(s, nls, full, n_known);
@@ -339,8 +337,7 @@ int optimize(rpgo_solver* s) {
           full.push_back(s->nfg[k + i]);
       full.insert(full.end(), s->temp_nfg.begin(), s->temp_nfg.end());
     }
-    GpuNls nls(s->dim, full, *s->store, sv.get(), s->st, s->p.linear_solver != RPGO_LINEAR_PCG);
-    nls.dev().coop_ctas = s->coop_ctas;
+    GpuNls nls(s->dim, full, *s->store, sv.get(), s->st, s->p.linear_solver != RPGO_LINEAR_PCG, s->coop_ctas);
     nls.optimize(lp, &st);
     if (st.failed) return RPGO_ERR_SOLVER;
     sv.write_back(nls);

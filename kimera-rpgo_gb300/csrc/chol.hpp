@@ -28,12 +28,20 @@ struct CholDev {
   DeviceBuffer<double> out;   // model change, status
   DeviceBuffer<double> Hs;    // H in the block layout of L (per linearisation)
   DeviceBuffer<double> dampS; // damping diagonal of the diagonal blocks, same layout
-  DeviceBuffer<int32_t> status;
+  DeviceBuffer<int32_t> status;  // pivot failure; a wait of the dataflow part ran out
+  // dataflow part (chol_plan.hpp) and the words its columns hand on: update
+  // products, forward and backward solutions
+  DeviceBuffer<int32_t> df_col, df_blk, df_dst, df_pre, df_row, df_trow;
+  DeviceBuffer<double> prod, ys, xs;
   cudaEvent_t ev[2] = {nullptr, nullptr};  // around each launch (kernel time)
   ~CholDev();
   void upload(CholPlan&& p, cudaStream_t st);
 };
 
+// CTAs of the solver's direct solve, and the widest level that its dataflow
+// part takes
+int chol_grid(const SolverDev& s);
+int chol_dataflow_cols(const SolverDev& s);
 // H and the damping diagonal in the block layout of L, from the linearised
 // system (Hd64, fH64, dampD); enqueued after every linearisation.
 // mask: a joint batch's variable control words (bit 0: graph in this round)
@@ -45,6 +53,9 @@ SolveOut chol_solve(SolverDev& s, CholDev& c, double lambda, cudaStream_t st);
 // chol_finish after the stream reached that point.
 void chol_enqueue(SolverDev& s, CholDev& c, double lambda, cudaStream_t st, double* host);
 SolveOut chol_finish(SolverDev& s, CholDev& c, const double* host);
+// throws when a solve's status word (0 solved, 1 a failed pivot, 2 a wait
+// between columns ran out) says that its kernel gave up
+void chol_check_status(double status);
 // Joint batch: enqueue one launch that solves every active system of the
 // batch b with its own damping; per-system model change and status land in
 // b.out (2 per system), the steps in s.delta.

@@ -1,7 +1,10 @@
 // Sparse block Cholesky solve of (H + lambda D) delta = -g on the GPU (FP64).
 //
-// One cooperative kernel per solve, 256 threads per CTA, one CTA per SM.
-// Phases are separated by grid barriers:
+// One cooperative kernel per solve, 256 threads per CTA, two CTAs per SM.
+// The wide levels of the elimination tree run as phases separated by grid
+// barriers (1 to 4 below); its narrow end, and a dense tail of one tile, run
+// as a dataflow between the forward and the backward phases (section
+// "dataflow part"). The phases:
 //  1. init: right-hand side in elimination order, padding of the dense tail;
 //  2. per elimination-tree level of the sparse columns (leaves first):
 //     (A) the level's tasks over all warps: for every block, its Hessian
@@ -74,6 +77,15 @@ struct CholArgs {
   // compacted per level, in plan order, ending at lvl_task_end / lvl_col_end)
   int b_compact;
   const int32_t *lvl_task_end, *lvl_col_end;
+  // dataflow part of the plan (chol_plan.hpp): columns, products from the
+  // columns before it, and the arrays whose words are handed from one column
+  // to the next (products, forward and backward solutions; df_stall: a wait
+  // ran out)
+  int df_level, df_cols, df_pre_n, df_tail, df_tail_blk;
+  size_t df_prod_n;
+  const int32_t *df_col, *df_blk, *df_dst, *df_pre, *df_row, *df_trow;
+  double *prod, *ys, *xs;
+  int32_t* df_stall;
 };
 
 // end of level l's tasks and columns (the compacted lists of a joint batch
@@ -1002,6 +1014,443 @@ __device__ void tail_backward_item(const CholArgs& a, double* yt, int k, TileSme
   __syncthreads();
 }
 
+// ------------------------------------------------------------------ dataflow part
+// The narrow end of the elimination tree (a few hundred columns per level and
+// fewer): a level barrier costs 1.1 us and a level took three of them, with
+// its work cut into two phases whose operands went through L2 each time
+// (3.7 us tasks, 6.0 us columns, 3.3 us backward per level on GB300, however
+// few columns the level has). Here every column belongs to one CTA, which
+// waits for exactly the words it needs: a product, an L block, a forward or a
+// backward solution. Such a word is reset to kEmpty before the first level
+// and carries its value from the moment it differs, so a hand-over is one
+// store and the load that the consumer issues anyway (no fence, flag or
+// atomic). A column computes the update products of its own blocks as soon
+// as they are solved; its ancestors only add them, in the order of the level
+// form (chunk by chunk), so the factor has the same bits.
+// Columns are taken in level order by CTAs that are all resident
+// (cooperative launch), so the lowest unfinished column never waits for one
+// that has no CTA. Every wait is bounded: after kDfSpins polls a CTA raises
+// df_stall, on which all waits end, and the host reports the solve as failed.
+// Waits are warp-wide: lanes that left a wait one by one would issue the
+// FP64 work behind it one by one (64 cycles each time).
+// Bound by the FP64 chain of a column (about 8,500 cycles from one level to
+// the next: six reciprocal square roots, 3,800 of them in all with their
+// products and FMAs, the row solves 1,400, the products 800, the hand-over
+// and the sums). Per solve, level form before -> now: 300 poses 264 -> 122
+// us, 5,000 poses 397 -> 214, 20,000 poses 617 -> 402, 50,000 poses 1,017 ->
+// 780.
+constexpr unsigned long long kEmpty = 0x7ffcd5c3a19b42e7ull;  // a NaN that no operation produces
+constexpr int kDfSpins = 1 << 21;
+constexpr int kDfMat = kThreads - 32;  // warps 0-6: the column's blocks; warp 7: its right-hand side
+
+__device__ __forceinline__ double ld_word(const double* p) {
+  double v;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_word(double* p, double v) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ bool is_empty(double v) {
+  return (unsigned long long)__double_as_longlong(v) == kEmpty;
+}
+// Words p[0], p[step], ... (n <= N of them, 0 in lanes without) as soon as
+// every lane of the warp has its own; all lanes of the warp call it.
+template <int N>
+__device__ __forceinline__ void ld_words(const CholArgs& a, const double* p, int step, int n, double (&v)[N]) {
+  int spins = 0;
+  while (true) {
+    bool all = true;
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = k < n ? ld_word(p + (size_t)k * step) : 0.0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) all = all && !is_empty(v[k]);
+    if (__all_sync(kFull, all)) return;
+    if ((++spins & 1023) == 0) {
+      if (spins >= kDfSpins) atomicExch(a.df_stall, 1);
+      if (__any_sync(kFull, *(volatile int32_t*)a.df_stall != 0)) return;
+    }
+  }
+}
+
+__device__ __forceinline__ bool df_on(const CholArgs& a, int j) {
+  return a.G == 0 || (a.b_act[a.b_sys[j]] & 1);
+}
+
+template <int D>
+struct DfSmem {
+  static constexpr int dd = D * D;
+  double S[(1 + kDfMaxBlocks) * dd];  // the column's blocks, then its solved blocks
+  double Lj[dd];                      // L_jj (lower part, reciprocal pivots)
+  double X[kTB][kTB + 1];             // the dense tail
+};
+
+__device__ __forceinline__ void df_mat_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kDfMat) : "memory"); }
+
+// v > 0 (false for NaN), from its bits: an FP64 comparison costs 64 cycles
+__device__ __forceinline__ bool positive(double v) {
+  const long long bits = __double_as_longlong(v);
+  return bits > 0 && bits <= 0x7ff0000000000000ll;
+}
+
+// Cholesky of S_jj by one warp, one lane per entry of the lower part: each
+// pivot costs a reciprocal square root, one product and one FMA on the FP64
+// pipe (64 cycles each whatever the lanes do), where a lane per row issues an
+// FMA per column. The same operations per entry as factor_diag.
+template <int D>
+__device__ __forceinline__ void df_factor(const CholArgs& a, int j, int lane, DfSmem<D>& s) {
+  constexpr int ntri = D * (D + 1) / 2;
+  int r = 0, c = lane < ntri ? lane : 0;
+  while (c > r) c -= ++r;
+  double v = s.S[r * D + c];
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    const double piv = __shfl_sync(kFull, v, k * (k + 3) / 2);
+    const bool pos = positive(piv);
+    ok = ok && pos;
+    const double il = rsqrt(pos ? piv : 1.0);
+    if (c == k) v = r == k ? il : v * il;
+    if (k + 1 < D) {
+      const double lr = __shfl_sync(kFull, v, r >= k ? r * (r + 1) / 2 + k : 0);
+      const double lc = __shfl_sync(kFull, v, c >= k ? c * (c + 1) / 2 + k : 0);
+      if (c > k) v = fma(-lr, lc, v);
+    }
+  }
+  if (!ok && lane == 0) set_fail(sys_status(a, j));
+  if (lane < ntri) {
+    s.Lj[r * D + c] = v;
+    a.Ldiag[(size_t)j * D * D + r * D + c] = v;
+  }
+}
+
+// Row r of a forward row sum over n entries of df_row from `row` on, by one
+// warp: run_task's order (G interleaved chains per chunk of 4 G entries).
+template <int D>
+__device__ __forceinline__ double df_row_sum(const CholArgs& a, int row, int n, int lane) {
+  constexpr int G = 32 / D, dd = D * D;
+  const int g = lane / D, r = lane % D;
+  double sum = 0.0;
+  for (int u0 = 0; u0 < n; u0 += 4 * G) {
+    const int nu = min(n - u0, 4 * G);
+    double acc = 0.0;
+    for (int u = 0; u < nu; u += G) {
+      const bool on = g < G && u + g < nu;
+      const int2 rb = reinterpret_cast<const int2*>(a.df_row)[row + u0 + (on ? u + g : 0)];
+      double Lq[D], yk[D];
+      ld_words<D>(a, a.L + (size_t)rb.x * dd + r * D, 1, on ? D : 0, Lq);
+      ld_words<D>(a, ((rb.y & 1) ? a.ys : a.y) + (size_t)(rb.y >> 1) * D, 1, on ? D : 0, yk);
+      if (on) {
+#pragma unroll
+        for (int k = 0; k < D; ++k) acc = fma(Lq[k], yk[k], acc);
+      }
+    }
+    __syncwarp();
+    const int ng = min(G, nu);
+    double tot = acc;
+#pragma unroll
+    for (int k = 1; k < G; ++k)
+      if (k < ng) tot += __shfl_sync(kFull, acc, (r + k * D) & 31);
+    sum += __shfl_sync(kFull, tot, r);
+  }
+  return sum;
+}
+
+// one column of the dataflow part by one CTA (w: its index in the part)
+template <int D>
+__device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
+  constexpr int G = 32 / D, dd = D * D;
+  const int4* rec = reinterpret_cast<const int4*>(a.df_col) + (size_t)w * (kDfColInts / 4);
+  const int4 r0 = rec[0], r1 = rec[1];
+  const int j = r0.x, p0 = r0.y, m = r0.z, blk0 = r0.w;
+  if (!df_on(a, j)) return;  // (CTA-uniform)
+  const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane / D, r = lane % D;
+  const int base = (g < G ? g : 0) * D;
+  if (wi < kDfMat / 32) {
+    const int mt = threadIdx.x;
+    // the destinations and Hessian entries of this thread's first products,
+    // ahead of the waits
+    const int4* dst = reinterpret_cast<const int4*>(a.df_dst) + r1.x;
+    const int nprod = m * (m + 1) / 2 * dd;
+    constexpr int kAhead = 2;
+    int4 d_rec[kAhead];
+    double d_H[kAhead];
+#pragma unroll
+    for (int x = 0; x < kAhead; ++x) {
+      const int it = mt + x * kDfMat;
+      d_rec[x] = it < nprod ? dst[it / dd] : make_int4(-1, 0, 0, 0);
+      d_H[x] = (d_rec[x].y & 1) ? block_H<D>(a, d_rec[x].y >> 2, d_rec[x].y & 2, it % dd / D, it % D) : 0.0;
+    }
+    // the column's blocks, a thread per entry: the products added in pair
+    // order within each chunk of G, the chunks in order (as they arrive, so
+    // that little is left to add after the last one), or the Hessian block
+    for (int i0 = 0; i0 < (1 + m) * dd; i0 += kDfMat) {
+      const int it = i0 + mt, b = it / dd, e = it % dd;
+      const bool on = it < (1 + m) * dd;
+      const int2 bl = on ? reinterpret_cast<const int2*>(a.df_blk)[blk0 + b] : make_int2(0, 0);
+      double v = (on && bl.y == 0) ? block_H<D>(a, p0 + b, b == 0, e / D, e % D) : 0.0;
+      constexpr int W = D == 6 ? 2 * G : G;  // words per wait
+      const int n = __reduce_max_sync(kFull, bl.y);
+      for (int u = 0; u < n; u += W) {
+        double x[W];
+        ld_words<W>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, x);
+#pragma unroll
+        for (int h = 0; h < W; h += G)
+          if (u + h < bl.y) {
+            double tot = x[h];
+#pragma unroll
+            for (int k = 1; k < G; ++k)
+              if (u + h + k < bl.y) tot += x[h + k];
+            v = u + h == 0 ? tot : v + tot;
+          }
+      }
+      __syncwarp();
+      if (on) s.S[it] = v;
+    }
+    df_mat_sync();
+    if (wi == 0) {
+      df_factor<D>(a, j, lane, s);
+      asm volatile("bar.arrive 2, 64;" ::: "memory");  // L_jj for the right-hand side's warp
+    }
+    df_mat_sync();
+    // L_ij = S_ij L_jj^-T, one row per lane group, one entry per lane
+    // (solve_offdiag's operations)
+    for (int rr0 = wi * G; rr0 < m * D; rr0 += kDfMat / 32 * G) {
+      const int rr = rr0 + g;
+      const bool on = g < G && rr < m * D;
+      double v = on ? s.S[dd + rr * D + r] : 0.0;
+#pragma unroll
+      for (int c = 0; c < D; ++c) {
+        const double x = __shfl_sync(kFull, v, base + c) * s.Lj[c * D + c];
+        if (r == c) v = x;
+        else if (r > c) v = fma(-x, s.Lj[r * D + c], v);
+      }
+      if (on) {
+        s.S[dd + rr * D + r] = v;
+        st_word(a.L + (size_t)(p0 + 1) * dd + rr * D + r, v);
+      }
+    }
+    df_mat_sync();
+    // the products of the column's blocks, to the blocks that add them
+    for (int x = 0, it = mt; it < nprod; ++x, it += kDfMat) {
+      const int4 d = x == 0 ? d_rec[0] : (x == 1 ? d_rec[1] : dst[it / dd]);
+      if (d.x < 0) continue;
+      const int e = it % dd, er = e / D, ec = e % D;
+      double acc = x == 0 ? d_H[0] : (x == 1 ? d_H[1] : ((d.y & 1) ? block_H<D>(a, d.y >> 2, d.y & 2, er, ec) : 0.0));
+      const double* A = s.S + (1 + d.w) * dd + er * D;
+      const double* B = s.S + (1 + d.z) * dd + ec * D;
+#pragma unroll
+      for (int k = 0; k < D; ++k) acc = fma(-A[k], B[k], acc);
+      st_word(a.prod + (size_t)d.x * dd + e, acc);
+    }
+  } else {
+    // right-hand side: the row sums, then y_j
+    const double sum = df_row_sum<D>(a, r1.y, r1.z, lane);
+    double b = a.y[(size_t)j * D + r] - sum;
+    asm volatile("bar.sync 2, 64;" ::: "memory");
+    double C[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) C[c] = c <= r ? s.Lj[r * D + c] : 0.0;
+    double yv = 0.0;
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      if (r == c) yv = b * C[c];
+      const double yc = __shfl_sync(kFull, yv, base + c);
+      if (r > c) b = fma(-C[c], yc, b);
+    }
+    if (g == 0) {
+      a.y[(size_t)j * D + r] = yv;
+      st_word(a.ys + (size_t)j * D + r, yv);
+    }
+  }
+  __syncthreads();  // s is reused by the CTA's next column
+}
+
+// The dense tail of one tile by one CTA, with the order of tail_block_cta,
+// smem_chol and the two substitutions: its blocks' products are added as
+// they arrive, so the phases and barriers that assembled, factored and
+// solved it after the last column (30 us) shrink to the factorisation.
+template <int D>
+__device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
+  constexpr int dd = D * D;
+  const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31, n = a.T * D;
+  double* yt = a.y + (size_t)a.ns * D;
+  double b = 0.0;  // warp 7: the right-hand side, a row per lane
+  if (wi < kDfMat / 32) {
+    const int ni = a.T * (a.T + 1) / 2 * dd;
+    for (int i0 = 0; i0 < ni; i0 += kDfMat) {
+      const int it = i0 + threadIdx.x, t = it / dd, e = it % dd, rr = e / D, cc = e % D;
+      const bool on = it < ni;
+      int bi = 0, bj = on ? t : 0;
+      while (bj > bi) bj -= ++bi;
+      const int2 bl = on ? reinterpret_cast<const int2*>(a.df_blk)[a.df_tail_blk + t] : make_int2(0, 0);
+      double v = 0.0;
+      if (on)
+        v = bi == bj ? gather_diag<D>(a, a.perm[a.ns + bi], rr, cc)
+                     : gather_offdiag<D>(a.fH64, a.ta_src, a.ta_ptr[t], a.ta_ptr[t + 1], rr, cc);
+      constexpr int W = 8;
+      const int np = __reduce_max_sync(kFull, bl.y);
+      for (int u = 0; u < np; u += W) {
+        double x[W];
+        ld_words<W>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, x);
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+          if (u + k < bl.y) v += x[k];
+      }
+      __syncwarp();
+      if (on) s.X[bi * D + rr][bj * D + cc] = v;
+    }
+    df_mat_sync();
+    for (int c = 0; c < n; ++c) {
+      // warp 0 takes the pivot and scales the column, all update the rest
+      if (wi == 0) {
+        const double piv = s.X[c][c];
+        const bool pos = positive(piv);
+        const int row = c + 1 + lane;
+        const double x = row < n ? s.X[row][c] : 0.0;
+        const double il = rsqrt(pos ? piv : 1.0);
+        if (row < n) s.X[row][c] = x * il;
+        __syncwarp();
+        if (lane == 0) {
+          if (!pos) set_fail(a.status);
+          s.X[c][c] = il;
+        }
+      }
+      df_mat_sync();
+      const int mr = n - c - 1;
+      for (int e = threadIdx.x; e < mr * (mr + 1) / 2; e += kDfMat) {
+        // entry e of the lower triangle, row by row
+        int r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+        while (r * (r + 1) / 2 > e) --r;
+        while ((r + 1) * (r + 2) / 2 <= e) ++r;
+        const int q = c + 1 + e - r * (r + 1) / 2;
+        r += c + 1;
+        s.X[r][q] = fma(-s.X[r][c], s.X[q][c], s.X[r][q]);
+      }
+      df_mat_sync();
+    }
+  } else {
+    for (int t = 0; t < a.T; ++t) {
+      const double sum = df_row_sum<D>(a, a.df_trow[2 * t], a.df_trow[2 * t + 1], lane);
+      if (lane / D == t) b = yt[lane] - sum;
+    }
+  }
+  __syncthreads();
+  if (wi == kDfMat / 32) {
+    double v = 0.0;
+    for (int c = 0; c < n; ++c) {
+      if (lane == c) v = b * s.X[c][c];
+      const double yc = __shfl_sync(kFull, v, c);
+      if (lane > c && lane < n) b = fma(-s.X[lane][c], yc, b);
+    }
+    b = v;
+    for (int c = n - 1; c >= 0; --c) {
+      if (lane == c) v = b * s.X[c][c];
+      const double xc = __shfl_sync(kFull, v, c);
+      if (lane < c) b = fma(-s.X[c][lane], xc, b);
+    }
+    if (lane < n) {
+      yt[lane] = v;
+      st_word(a.xs + (size_t)a.ns * D + lane, v);
+    }
+  }
+}
+
+// products of the pairs that come from the columns before the dataflow part
+// (all factored), a product per lane group
+template <int D>
+__device__ void df_pre_products(const CholArgs& a, int gw, int nw, int lane) {
+  constexpr int G = 32 / D, dd = D * D;
+  const int g = lane / D, r = lane % D;
+  for (int w = gw * G; w < a.df_pre_n; w += nw * G) {
+    if (g >= G || w + g >= a.df_pre_n) continue;
+    const int4 d = reinterpret_cast<const int4*>(a.df_pre)[w + g];
+    if (!df_on(a, a.blk_col[d.w >> 2])) continue;
+    const double* A = a.L + (size_t)d.y * dd + r * D;
+    const double* B = a.L + (size_t)d.z * dd;
+    double ar[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) ar[k] = A[k];
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      double acc = (d.w & 1) ? block_H<D>(a, d.w >> 2, d.w & 2, r, c) : 0.0;
+#pragma unroll
+      for (int k = 0; k < D; ++k) acc = fma(-ar[k], B[c * D + k], acc);
+      st_word(a.prod + (size_t)d.x * dd + r * D + c, acc);
+    }
+  }
+}
+
+// empties every word that a column of the dataflow part hands on
+template <int D>
+__device__ void df_reset(const CholArgs& a, int gt, int gs) {
+  constexpr int dd = D * D;
+  const double e = __longlong_as_double((long long)kEmpty);
+  for (size_t k = gt; k < a.df_prod_n * dd; k += gs) st_word(a.prod + k, e);
+  for (int k = gt; k < a.N * D; k += gs) {
+    st_word(a.ys + k, e);
+    st_word(a.xs + k, e);
+  }
+  const int lane = gt & 31;
+  for (int w = gt >> 5; w < a.df_cols; w += gs >> 5) {
+    const int p0 = a.df_col[(size_t)w * kDfColInts + 1], m = a.df_col[(size_t)w * kDfColInts + 2];
+    for (int k = lane; k < m * dd; k += 32) st_word(a.L + (size_t)(p0 + 1) * dd + k, e);
+  }
+}
+
+// Backward substitution of the dataflow part, a warp per column from the
+// last one down (backward_warp_core's operations); a CTA takes the columns
+// that it factored, so only the solutions above them are waited for.
+template <int D>
+__device__ void df_backward(const CholArgs& a, int lane) {
+  constexpr int G = 32 / D, dd = D * D;
+  const int g = lane / D, r = lane % D;
+  const int base = (g < G ? g : 0) * D;
+  const int own = a.df_cols > (int)blockIdx.x ? (a.df_cols - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  for (int k = own - 1 - (int)(threadIdx.x >> 5); k >= 0; k -= kWarps) {
+    const int32_t* rec = a.df_col + (size_t)((int)blockIdx.x + k * (int)gridDim.x) * kDfColInts;
+    const int j = rec[0], q0 = rec[1] + 1, q1 = q0 + rec[2];
+    if (!df_on(a, j)) continue;  // (warp-uniform)
+    const double yj = a.y[(size_t)j * D + r];
+    double Lc[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) Lc[c] = c >= r ? a.Ldiag[(size_t)j * dd + c * D + r] : 0.0;
+    double acc = 0.0;
+    for (int q = q0; q < q1; q += G) {
+      const bool on = g < G && q + g < q1;
+      const int row = on ? a.blk_row[q + g] : 0;
+      const double* B = a.L + (size_t)(q + g) * dd + r;
+      double Bv[D], xv[D];
+#pragma unroll
+      for (int i = 0; i < D; ++i) Bv[i] = on ? B[i * D] : 0.0;
+      ld_words<D>(a, (row < a.ns || a.df_tail ? a.xs : a.y) + (size_t)row * D, 1, on ? D : 0, xv);
+      if (on) {
+#pragma unroll
+        for (int i = 0; i < D; ++i) acc = fma(Bv[i], xv[i], acc);
+      }
+    }
+    __syncwarp();
+    const int ng = min(G, q1 - q0);
+    double tot = acc;
+#pragma unroll
+    for (int i = 1; i < G; ++i)
+      if (i < ng) tot += __shfl_sync(kFull, acc, (r + i * D) & 31);
+    double b = yj - tot;
+    double x = 0.0;
+#pragma unroll
+    for (int c = D - 1; c >= 0; --c) {
+      if (r == c) x = b * Lc[c];
+      const double xc = __shfl_sync(kFull, x, base + c);
+      if (r < c) b = fma(-Lc[c], xc, b);
+    }
+    if (g == 0) {
+      a.y[(size_t)j * D + r] = x;
+      st_word(a.xs + (size_t)j * D + r, x);
+    }
+  }
+}
+
 __device__ __forceinline__ double cta_sum(double v, double* sh) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -1017,7 +1466,10 @@ __device__ __forceinline__ double cta_sum(double v, double* sh) {
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
   cg::grid_group grid = cg::this_grid();
-  __shared__ TileSmem sm;
+  // (the dataflow part and the other phases use it in turn, a barrier between)
+  __shared__ __align__(16) unsigned char smem[sizeof(TileSmem) > sizeof(DfSmem<D>) ? sizeof(TileSmem)
+                                                                                  : sizeof(DfSmem<D>)];
+  TileSmem& sm = *reinterpret_cast<TileSmem*>(smem);
   __shared__ double shr[kThreads / 32];
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
@@ -1032,7 +1484,8 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
   double* yt = a.y + (size_t)a.ns * D;
 
   // 1. init
-  if (gt == 0) *a.status = 0;
+  if (gt == 0) *a.status = *a.df_stall = 0;
+  if (a.df_cols > 0) df_reset<D>(a, gt, gs);
   for (int k = gt; k < a.G; k += gs) a.b_status[k] = 0;
   for (int k = gt; k < n; k += gs) {
     const int pos = k / D, r = k % D;
@@ -1058,7 +1511,7 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
   const int team_slot = (wi - 1) >> 1;
   const int team_w = team_slot * (int)gridDim.x + (int)blockIdx.x;
   bool task_ready = false;  // sm.task[wi][lane] holds this warp's first task of level l
-  for (int l = 0; l < a.levels; ++l) {
+  for (int l = 0; l < a.df_level; ++l) {
     const int t0 = a.lvl_task_ptr[l], t1 = task_end(a, l);
     const int c0 = a.lvl_col_ptr[l], nc = col_end(a, l) - c0;
     const bool narrow = nc < kGroupModeItems * nw && nc <= 2 * (int)gridDim.x;
@@ -1102,7 +1555,7 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
     // the warp's first task of the next level (narrow task phases), ahead of
     // the barrier, through shared memory
     task_ready = false;
-    if (l + 1 < a.levels) {
+    if (l + 1 < a.df_level) {
       const int u0 = a.lvl_task_ptr[l + 1], u1 = task_end(a, l + 1);
       if (u1 > u0 && u1 - u0 < kGroupModeItems * nw && u0 + gw < u1) {
         task_ahead<D>(a, u0 + gw, lane, sm.task[wi][lane]);
@@ -1111,18 +1564,25 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
     }
     grid.sync();
   }
+  if (a.df_cols > 0) {
+    df_pre_products<D>(a, gw, nw, lane);
+    DfSmem<D>& ds = *reinterpret_cast<DfSmem<D>*>(smem);
+    for (int w = blockIdx.x; w < a.df_cols; w += gridDim.x) df_column<D>(a, w, ds);
+    if (a.df_tail && (int)blockIdx.x == a.df_cols % (int)gridDim.x) df_tail<D>(a, ds);
+    if (!a.df_tail) grid.sync();
+  }
 
   // 3. dense tail: its blocks (one CTA each) and the row sums of its
   // right-hand side (one warp each, on the CTAs after the blocks'), then the
   // tiles
-  {
+  if (!a.df_tail) {
     const int nts = a.T * (a.T + 1) / 2, ntr = a.ttask_ptr[a.T];
     for (int b = blockIdx.x; b < nts; b += gridDim.x) tail_block_cta<D>(a, b, sm);
     for (int w = gw; w < nts + ntr; w += nw)
       if (w >= nts) tail_row_task<D>(a, w - nts, lane);
+    grid.sync();
   }
-  grid.sync();
-  const int nT = a.n_tiles;
+  const int nT = a.df_tail ? 0 : a.n_tiles;  // (df_tail: the tail is solved)
   if (nT == 1) {
     // a single tile: one CTA takes the tail's right-hand side, its
     // factorisation and both substitutions, in one phase
@@ -1168,7 +1628,11 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
   // the warp's column of the next level is loaded ahead of each barrier
   BackAhead back;
   int back_l = -1;  // the level whose column `back` holds
-  for (int l = a.levels - 1; l >= 0; --l) {
+  if (a.df_cols > 0) {
+    df_backward<D>(a, lane);
+    grid.sync();
+  }
+  for (int l = a.df_level - 1; l >= 0; --l) {
     const int c0 = a.lvl_col_ptr[l], nc = col_end(a, l) - c0;
     if (nc <= (kWarps - 1) * (int)gridDim.x) {
       if (gw < nc) {
@@ -1225,7 +1689,7 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
       }
       if (lane == 0) {
         a.b_out[2 * sy] = -0.5 * sg + 0.5 * a.b_lam[sy] * sq;
-        a.b_out[2 * sy + 1] = (double)atomicAdd(a.b_status + sy, 0);
+        a.b_out[2 * sy + 1] = *(volatile int32_t*)a.df_stall ? 2.0 : (double)atomicAdd(a.b_status + sy, 0);
       }
     }
     return;
@@ -1260,7 +1724,7 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
     if (threadIdx.x == 0) {
       a.out[0] = -0.5 * sg + 0.5 * a.lam * sq;
       // every block's pivot failures were flagged before the last barrier
-      a.out[1] = (double)atomicAdd(a.status, 0);
+      a.out[1] = *(volatile int32_t*)a.df_stall ? 2.0 : (double)atomicAdd(a.status, 0);
     }
   }
 }
@@ -1428,7 +1892,18 @@ void CholDev::upload(CholPlan&& p, cudaStream_t st) {
   Ldd.resize(std::max<size_t>(1, (size_t)plan.n_tiles * kTB * kTB));
   y.resize((size_t)plan.n_sparse * plan.d + ntp + 1);
   out.resize(4);
-  status.resize(1);
+  status.resize(2);
+  df_col.upload(plan.df_col, st);
+  df_blk.upload(plan.df_blk, st);
+  df_dst.upload(plan.df_dst, st);
+  df_pre.upload(plan.df_pre, st);
+  df_row.upload(plan.df_row, st);
+  df_trow.upload(plan.df_trow, st);
+  if (!plan.df_col.empty()) {
+    prod.resize(std::max<size_t>(1, (size_t)plan.df_products * dd));
+    ys.resize((size_t)plan.N * plan.d);
+    xs.resize((size_t)plan.N * plan.d);
+  }
 }
 
 CholDev::~CholDev() {
@@ -1455,7 +1930,7 @@ void chol_block_hessian(SolverDev& s, CholDev& c, cudaStream_t st, const uint8_t
 // CTAs of the cooperative solve: every co-resident CTA (two per SM at 256
 // threads x 128 registers: twice the warps per SM to hide the latency of the
 // wide levels' loads), or the caller's budget
-static int chol_grid(const SolverDev& s) {
+int chol_grid(const SolverDev& s) {
   static const int per_sm[2] = {
       [] {
         int n = 0;
@@ -1470,6 +1945,15 @@ static int chol_grid(const SolverDev& s) {
   const int most = device_sm_count() * per_sm[s.dim == 3 ? 1 : 0];
   return s.coop_ctas > 0 ? std::min(s.coop_ctas, most) : most;
 }
+
+// A level in the dataflow part takes about 4 us per column of its busiest
+// CTA, one in the level form about 11 us and what its width adds. Widest
+// level swept at 1 / 2 / 4 / 8 columns per CTA: 304 CTAs, 5,000 poses 236 /
+// 220 / 214 / 215 us per solve, 20,000 poses 439 / 417 / 402 / 403, 50,000
+// poses 822 / 797 / 780 / 775 (and 513 and 845 at 20 columns per CTA); batches
+// on 76 CTAs each, 16 graphs of 200 to 2,000 poses: 124 (2) / 121 (4) / 122
+// (8) / 130 (16) ms; on 19 CTAs each: 144 (8) / 157 (16) / 197 ms (32).
+int chol_dataflow_cols(const SolverDev& s) { return 4 * chol_grid(s); }
 
 // kernel arguments of one solve (one system; the joint batch adds its own)
 static CholArgs make_args(SolverDev& s, CholDev& c, double lambda) {
@@ -1490,6 +1974,22 @@ static CholArgs make_args(SolverDev& s, CholDev& c, double lambda) {
   a.b_out = a.b_term = nullptr;
   a.b_compact = 0;
   a.lvl_task_end = a.lvl_col_end = nullptr;
+  a.df_level = p.df_level;
+  a.df_cols = (int)(p.df_col.size() / kDfColInts);
+  a.df_pre_n = (int)(p.df_pre.size() / 4);
+  a.df_prod_n = (size_t)p.df_products;
+  a.df_tail = p.df_tail;
+  a.df_tail_blk = p.df_tail_blk;
+  a.df_col = c.df_col.get();
+  a.df_blk = c.df_blk.get();
+  a.df_dst = c.df_dst.get();
+  a.df_pre = c.df_pre.get();
+  a.df_row = c.df_row.get();
+  a.df_trow = c.df_trow.get();
+  a.prod = c.prod.get();
+  a.ys = c.ys.get();
+  a.xs = c.xs.get();
+  a.df_stall = c.status.get() + 1;
   return a;
 }
 
@@ -1517,6 +2017,10 @@ void chol_enqueue(SolverDev& s, CholDev& c, double lambda, cudaStream_t st, doub
   RPGO_CUDA(cudaMemcpyAsync(host, c.out.get(), 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
 }
 
+void chol_check_status(double status) {
+  if (status == 2.0) throw CudaError("direct solve: a wait between columns ran out");
+}
+
 SolveOut chol_finish(SolverDev& s, CholDev& c, const double* host) {
   SolveOut o;
   if (s.N == 0) {
@@ -1532,6 +2036,7 @@ SolveOut chol_finish(SolverDev& s, CholDev& c, const double* host) {
   kernel_times().chol_bytes += p.bytes;
   kernel_times().chol_levels = c.levels;
   kernel_times().chol_tail = p.T;
+  chol_check_status(host[1]);
   o.lin_change = host[0];
   o.ok = host[1] == 0.0 ? 1 : 0;
   return o;
@@ -1558,19 +2063,18 @@ SolveOut chol_solve(SolverDev& s, CholDev& c, double lambda, cudaStream_t st) {
     RPGO_LAUNCHED();
     ms = timer.elapsed_ms();
   }
-  double h = 0.0;
-  int32_t status = 0;
-  RPGO_CUDA(cudaMemcpyAsync(&h, c.out.get(), sizeof(double), cudaMemcpyDeviceToHost, st));
-  RPGO_CUDA(cudaMemcpyAsync(&status, c.status.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  double h[2] = {0.0, 0.0};  // model change, status
+  RPGO_CUDA(cudaMemcpyAsync(h, c.out.get(), sizeof(h), cudaMemcpyDeviceToHost, st));
   RPGO_CUDA(cudaStreamSynchronize(st));
+  chol_check_status(h[1]);
   kernel_times().chol_ms += ms;
   kernel_times().chol_launches += 1;
   kernel_times().chol_flops += p.flops;
   kernel_times().chol_bytes += p.bytes;
   kernel_times().chol_levels = c.levels;
   kernel_times().chol_tail = p.T;
-  o.lin_change = h;
-  o.ok = status == 0 ? 1 : 0;
+  o.lin_change = h[0];
+  o.ok = h[1] == 0.0 ? 1 : 0;
   o.cg_iterations = 0;
   o.rel_residual = 0.0;
   return o;

@@ -696,6 +696,7 @@ CholPlan make_chol_plan(int N, int d, const std::vector<int32_t>& kind, const st
               + 2.0 * factor        // read by the forward and the backward substitution
               + 8.0 * d * N * 6.0;  // gradient, damping, rhs / solution, step, model change
   }
+  p.df_level = p.levels();
   return p;
 }
 
@@ -830,7 +831,89 @@ CholPlan merge_chol_plans(const std::vector<CholPlan>& plans, const std::vector<
   u.ta_ptr.assign(1, 0);
   u.trow_ptr.assign(1, 0);
   u.ttask_ptr.assign(1, 0);
+  u.df_level = u.levels();
   return u;
+}
+
+void add_dataflow(CholPlan& p, int max_cols) {
+  const int ns = p.n_sparse, L = p.levels();
+  auto fits = [&](int j) {
+    if (p.col_ptr[j + 1] - p.col_ptr[j] - 1 > kDfMaxBlocks) return false;
+    int chunks = 0;
+    for (int q = p.col_ptr[j]; q < p.col_ptr[j + 1]; ++q) chunks += p.btask[2 * q + 1];
+    return chunks <= kDfMaxChunks;
+  };
+  int l0 = L;
+  while (l0 > 0 && p.lvl_col_ptr[l0] - p.lvl_col_ptr[l0 - 1] <= max_cols &&
+         std::all_of(p.lvl_cols.begin() + p.lvl_col_ptr[l0 - 1], p.lvl_cols.begin() + p.lvl_col_ptr[l0], fits))
+    --l0;
+  p.df_level = l0;
+  if (l0 == L) return;
+  const int w0 = p.lvl_col_ptr[l0];
+  std::vector<uint8_t> in_df(ns, 0);
+  for (int w = w0; w < ns; ++w) in_df[p.lvl_cols[w]] = 1;
+  p.df_tail = p.n_tiles <= 1;
+  for (int t = 0; t < p.n_tail_blocks() && p.df_tail; ++t)
+    if (p.tupd_ptr[t + 1] - p.tupd_ptr[t] > tail_slots(p.d)) p.df_tail = 0;
+  // products and rows of the part's columns, then of the tail
+  int np = 0;
+  auto add_block = [&](int pairs) {
+    p.df_blk.push_back(np);
+    p.df_blk.push_back(pairs);
+    np += pairs;
+    return np - pairs;
+  };
+  auto add_rows = [&](const std::vector<int32_t>& ptr, const std::vector<int32_t>& blk, int r) {
+    for (int u = ptr[r]; u < ptr[r + 1]; ++u) {
+      p.df_row.push_back(blk[2 * u]);
+      p.df_row.push_back(blk[2 * u + 1] << 1 | in_df[blk[2 * u + 1]]);
+    }
+    return ptr[r + 1] - ptr[r];
+  };
+  std::vector<int32_t> base(p.n_blocks(), -1), dst0(ns, 0);  // first product of a block, df_dst entry of a column
+  int nd = 0;
+  for (int w = w0; w < ns; ++w) {
+    const int j = p.lvl_cols[w], p0 = p.col_ptr[j], m = p.col_ptr[j + 1] - p0 - 1;
+    const int blk0 = (int)p.df_blk.size() / 2, row0 = (int)p.df_row.size() / 2;
+    for (int q = p0; q <= p0 + m; ++q) base[q] = add_block(p.upd_ptr[q + 1] - p.upd_ptr[q]);
+    const int32_t rec[kDfColInts] = {j, p0, m, blk0, nd, row0, add_rows(p.row_ptr, p.row_blk, j), 0};
+    p.df_col.insert(p.df_col.end(), rec, rec + kDfColInts);
+    dst0[j] = nd;
+    for (int a = 0; a < m; ++a)
+      for (int b = a; b < m; ++b, ++nd) p.df_dst.insert(p.df_dst.end(), {-1, 0, a, b});
+  }
+  // the product of pair (pb, pa) = (larger row, smaller row) of one column
+  auto place = [&](int pb, int pa, int product, int code) {
+    const int k = p.blk_col[pa];
+    if (!in_df[k]) {
+      p.df_pre.insert(p.df_pre.end(), {product, pb, pa, code});
+      return;
+    }
+    const int m = p.col_ptr[k + 1] - p.col_ptr[k] - 1, a = pa - p.col_ptr[k] - 1, b = pb - p.col_ptr[k] - 1;
+    int32_t* d = &p.df_dst[(size_t)4 * (dst0[k] + a * m - a * (a - 1) / 2 + (b - a))];
+    d[0] = product;
+    d[1] = code;
+  };
+  for (int w = w0; w < ns; ++w) {
+    const int p0 = p.col_ptr[p.lvl_cols[w]], p1 = p.col_ptr[p.lvl_cols[w] + 1];
+    for (int q = p0; q < p1; ++q)
+      for (int u = p.upd_ptr[q]; u < p.upd_ptr[q + 1]; ++u)
+        place(p.upd_src[2 * u], p.upd_src[2 * u + 1], base[q] + (u - p.upd_ptr[q]),
+              q << 2 | (q == p0 ? 2 : 0) | (u == p.upd_ptr[q] ? 1 : 0));
+  }
+  if (p.df_tail) {
+    p.df_tail_blk = (int)p.df_blk.size() / 2;
+    for (int t = 0; t < p.n_tail_blocks(); ++t) {
+      const int b = add_block(p.tupd_ptr[t + 1] - p.tupd_ptr[t]);
+      for (int u = p.tupd_ptr[t]; u < p.tupd_ptr[t + 1]; ++u)
+        place(p.tupd_src[2 * u], p.tupd_src[2 * u + 1], b + (u - p.tupd_ptr[t]), 0);
+    }
+    for (int t = 0; t < p.T; ++t) {
+      const int row0 = (int)p.df_row.size() / 2;
+      p.df_trow.insert(p.df_trow.end(), {row0, add_rows(p.trow_ptr, p.trow_blk, t)});
+    }
+  }
+  p.df_products = np;
 }
 
 }  // namespace rpgo

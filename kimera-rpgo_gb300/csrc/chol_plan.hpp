@@ -19,6 +19,13 @@
 
 namespace rpgo {
 
+// limits of a dataflow column: off-diagonal blocks, update chunks of its
+// blocks; ints per column in df_col
+constexpr int kDfMaxBlocks = 15, kDfMaxChunks = 64, kDfColInts = 8;
+// lane groups of a CTA of the solve kernel: the dense tail's blocks add their
+// update pairs in this many interleaved chains
+constexpr int tail_slots(int d) { return 8 * (32 / d); }
+
 struct CholPlan {
   int N = 0;             // variables (block columns)
   int d = 6;             // block size
@@ -68,6 +75,30 @@ struct CholPlan {
   // column) pairs
   std::vector<int32_t> row_ptr, row_blk;
   std::vector<int32_t> trow_ptr, trow_blk;
+  // Dataflow part: the columns of levels [df_level, levels()), in the order
+  // of lvl_cols, whose factorisation hands its update products on as it goes
+  // instead of waiting for a level barrier. A product is L[a] L[b]^T of one
+  // update pair whose target block is in such a column (the block's first
+  // pair carries the Hessian block) or, with df_tail set, in the dense tail;
+  // the products of a block are numbered consecutively in pair order. df_tail:
+  // the tail has at most one tile and none of its blocks more pairs than
+  // tail_slots.
+  //  df_col: kDfColInts ints per column: position, first block, off-diagonal
+  //    blocks m, first entry of df_blk, first entry of df_dst, first entry of
+  //    df_row, entries of df_row, 0;
+  //  df_blk: (first product, pairs) per block of a column (diagonal first),
+  //    then per tail block;
+  //  df_dst: per pair (a, b), a <= b, of the column's off-diagonal blocks, in
+  //    the order of the update lists: (product, or -1 for a tail block
+  //    without df_tail; target block << 2 | diagonal << 1 | first pair, 0 for
+  //    a tail block; a; b);
+  //  df_pre: products whose pair comes from a column before df_level:
+  //    (product, block a, block b, target code as in df_dst);
+  //  df_row: the row list of each column, then of each tail block row: (block,
+  //    column << 1 | column in the dataflow part);
+  //  df_trow: (first entry of df_row, entries) per tail block row.
+  int df_level = 0, df_products = 0, df_tail = 0, df_tail_blk = 0;  // df_tail_blk: first tail entry of df_blk
+  std::vector<int32_t> df_col, df_blk, df_dst, df_pre, df_row, df_trow;
   int levels() const { return (int)lvl_col_ptr.size() - 1; }
   int n_blocks() const { return (int)blk_row.size(); }
   int n_tail_blocks() const { return T * (T + 1) / 2; }
@@ -90,5 +121,11 @@ CholPlan make_chol_plan(int N, int d, const std::vector<int32_t>& kind, const st
 // every plan's level l, ordered as make_chol_plan orders a level. Each
 // system's operations are those of its own plan.
 CholPlan merge_chol_plans(const std::vector<CholPlan>& plans, const std::vector<int32_t>& foff);
+
+// Fills in the plan's dataflow part (empty until then): the levels from the
+// first one after which every level has at most max_cols columns and every
+// column is within the limits. It changes the schedule only, not the order of
+// any sum.
+void add_dataflow(CholPlan& p, int max_cols);
 
 }  // namespace rpgo

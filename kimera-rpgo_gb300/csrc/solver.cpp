@@ -11,8 +11,9 @@
 namespace rpgo {
 
 GpuNls::GpuNls(int dim, const std::vector<FactorRec>& graph, const FactorStore& store, const ValueStore& values,
-               cudaStream_t st, bool direct)
+               cudaStream_t st, bool direct, int coop_ctas)
     : dim_(dim), st_(st) {
+  s_.coop_ctas = coop_ctas;
   const int stride = dim == 3 ? 12 : 4, d = dim == 3 ? 6 : 3;
   std::unordered_map<uint64_t, int> index;
   index.reserve(values.size());

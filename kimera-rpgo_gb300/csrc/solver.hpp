@@ -39,7 +39,7 @@ class GpuNls {
   // informations and initial values gathered on the device from the stores
   // direct: sparse Cholesky steps (else whole-GPU PCG)
   GpuNls(int dim, const std::vector<FactorRec>& graph, const FactorStore& store, const ValueStore& values,
-         cudaStream_t st, bool direct = true);
+         cudaStream_t st, bool direct = true, int coop_ctas = 0);
   void set_weights(const std::vector<double>& w);
   // LM / GN from the initial values (from_current: from the estimate in
   // dev().x); result left in dev().x

@@ -684,6 +684,7 @@ void solver_upload(SolverDev& s, int dim, const std::vector<int32_t>& kind, cons
   const int d = s.d, dd = d * d, F = s.F;
   // the direct solve's plan (host work only) is built on its own thread while
   // the lists below are built and uploaded
+  const int df_cols = direct && N > 0 ? chol_dataflow_cols(s) : 0;
   CholPlan plan;
   std::exception_ptr plan_err;
   struct Joiner {
@@ -696,6 +697,7 @@ void solver_upload(SolverDev& s, int dim, const std::vector<int32_t>& kind, cons
     planner.t = std::thread([&] {
       try {
         plan = make_chol_plan(N, d, kind, vi, vj);
+        add_dataflow(plan, df_cols);
       } catch (...) {
         plan_err = std::current_exception();
       }
@@ -802,7 +804,10 @@ void solver_upload(SolverDev& s, int dim, const std::vector<int32_t>& kind, cons
   if (direct && N > 0) {
     if (planner.t.joinable()) planner.t.join();
     if (plan_err) std::rethrow_exception(plan_err);
-    if (given) plan = std::move(*given);
+    if (given) {
+      plan = std::move(*given);
+      add_dataflow(plan, df_cols);
+    }
     const double ntp = (double)plan.n_tiles * plan.tile;
     const double bytes = 8.0 * dd * (plan.n_blocks() + plan.n_sparse) + 8.0 * ntp * ntp +
                          4.0 * (plan.upd_src.size() + plan.tupd_src.size());
