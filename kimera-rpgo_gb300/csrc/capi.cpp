@@ -1118,10 +1118,10 @@ int rpgo_trajectory_scan_dev(int32_t dim, int32_t mode, int64_t count, const int
   if ((dim != 2 && dim != 3) || (mode != 0 && mode != 1) || count < 0) return RPGO_ERR_ARG;
   AllocStreamScope scope((cudaStream_t)stream);
   return guarded([&] {
-    DeviceBuffer<double> rec, cov;
+    DeviceBuffer<double> rec;
     DeviceBuffer<uint8_t> rot;
     TrajView tv{traj_pose, traj_cov, traj_node, traj_rot_info};
-    launch_traj_scan(dim, mode, count, src, dst, delta_pose, delta_cov, tv, rec, cov, rot, (cudaStream_t)stream);
+    launch_traj_scan(dim, mode, count, src, dst, delta_pose, delta_cov, tv, rec, rot, (cudaStream_t)stream);
     RPGO_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     return (int)RPGO_OK;
   });

@@ -336,7 +336,7 @@ bool PcmEngine::remove_outliers(const std::vector<FactorRec>& new_factors, const
     gather_rows((int64_t)orows.size(), d_rows_.get(), store.meas(), stride_, d_dpose_.get(), st_);
     gather_rows((int64_t)orows.size(), d_rows_.get(), store.cov(), d_ * d_, d_dcov_.get(), st_);
     launch_traj_scan(cfg_.dim, cfg_.mode, (int64_t)src.size(), d_src_.get(), d_dst_.get(), d_dpose_.get(),
-                     d_dcov_.get(), view(), scratch_rec_, scratch_cov_, scratch_rot_, st_);
+                     d_dcov_.get(), view(), scratch_rec_, scratch_rot_, st_);
   }
   if (!lcs.empty()) {
     // ---- odometry consistency of intra-robot closures (Pcm.h:455-465, 604-629)

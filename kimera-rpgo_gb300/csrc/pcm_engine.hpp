@@ -166,7 +166,7 @@ class PcmEngine {
   // scratch
   DeviceBuffer<int32_t> d_src_, d_dst_;
   DeviceBuffer<int64_t> d_rows_;
-  DeviceBuffer<double> d_dpose_, d_dcov_, scratch_rec_, scratch_cov_;
+  DeviceBuffer<double> d_dpose_, d_dcov_, scratch_rec_;
   DeviceBuffer<uint8_t> scratch_rot_, d_ok_;
   DeviceBuffer<uint32_t> lower_scratch_;
   CliqueWorkspace clique_ws_;

@@ -227,393 +227,271 @@ __device__ __forceinline__ bool check_u(const PWN<DIM>& u, double th0, double th
 }
 
 // ------------------------------------------------------------------ K0
-// Exact per-element pieces of PWC::compose for one lane.
-__device__ __forceinline__ double p3_compose_elem(const double* A, const double* B, int e) {
-  // A, B: 12-double pose records (R row-major, t)
-  if (e < 9) {
-    const int i = e / 3, j = e % 3;
-    return dot3e(A[3 * i], A[3 * i + 1], A[3 * i + 2], B[j], B[3 + j], B[6 + j]);
-  }
-  const int i = e - 9;
-  double acc = fmad(A[3 * i], B[9], A[9 + i]);
-  acc = fmad(A[3 * i + 1], B[10], acc);
-  return fmad(A[3 * i + 2], B[11], acc);
-}
-__device__ __forceinline__ double p2_compose_elem(const double* A, const double* B, int e) {
-  // (c, s, x, y)
-  switch (e) {
-    case 0: return fmad(A[0], B[0], -mul(A[1], B[1]));
-    case 1: return fmad(A[1], B[0], mul(A[0], B[1]));
-    case 2: return add(A[2], fmad(A[0], B[2], -mul(A[1], B[3])));
-    default: return add(A[3], fmad(A[1], B[2], mul(A[0], B[3])));
-  }
-}
-
-// Per-odometry-factor constants: the measurement as an uncertain pose
-// (GeometryUtils.h:91-115) and the pieces of Ad(Delta^-1).
+// Per-odometry-factor constants of the covariance walk, one record per step:
+// Ad(Delta^-1) (3D: its blocks R and K, 9 each; 2D: 9) and the lower triangle
+// of the measurement's covariance as an uncertain pose (GeometryUtils.h:91-115).
+template <int DIM>
+struct ScanRec {
+  static constexpr int ad = DIM == 3 ? 18 : 9, d = DIM == 3 ? 6 : 3, n = ad + d * (d + 1) / 2;
+};
 template <int DIM>
 __global__ void k_odom_prep(int64_t count, const double* __restrict__ dpose, const double* __restrict__ dcov,
-                            double* __restrict__ inv_rec, double* __restrict__ cov_out, uint8_t* __restrict__ rot_out) {
+                            double* __restrict__ rec, uint8_t* __restrict__ rot_out) {
   using L = Lie<DIM>;
+  using C = ScanRec<DIM>;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= count) return;
   PWC<DIM> z;
   z.from_factor(dpose + k * L::stride, dcov + k * L::d * L::d);
-  for (int i = 0; i < L::d * L::d; ++i) cov_out[k * L::d * L::d + i] = z.cov[i];
   rot_out[k] = z.rot ? 1 : 0;
+  double* r = rec + k * C::n;
   typename L::Pose inv;
   L::inverse(z.pose, inv);
   if constexpr (DIM == 3) {
     double K[9];
     p3_adjoint_K(inv, K);
-    double* r = inv_rec + k * 21;
     for (int i = 0; i < 9; ++i) r[i] = inv.R[i];
     for (int i = 0; i < 9; ++i) r[9 + i] = K[i];
-    for (int i = 0; i < 3; ++i) r[18 + i] = inv.t[i];
   } else {
     double A[9];
     p2_adjoint(inv, A);
-    double* r = inv_rec + k * 9;
     for (int i = 0; i < 9; ++i) r[i] = A[i];
   }
+  for (int i = 0, e = C::ad; i < C::d; ++i)
+    for (int j = 0; j <= i; ++j, ++e) r[e] = z.cov[C::d * i + j];
 }
 
-// One warp walks the odometry list in order. The step constants of step k+1
-// (odometry pose, Ad(Delta^-1) pieces, covariance, indices) are loaded into
-// registers while step k computes and land in shared memory at its end, so
-// the walk waits on memory only when a chain restarts from an older pose.
-template <int DIM, int MODE>
-__global__ void __launch_bounds__(32) k_traj_scan(int64_t count, const int32_t* __restrict__ src,
-                                                  const int32_t* __restrict__ dst, const double* __restrict__ dpose,
-                                                  const double* __restrict__ inv_rec,
-                                                  const double* __restrict__ dcov_p,
-                                                  const uint8_t* __restrict__ drot, TrajView tr) {
-  using L = Lie<DIM>;
-  constexpr int d = L::d, st = L::stride, dd = d * d;
-  constexpr int REC = (DIM == 3) ? 21 : 9;
-  constexpr int NC = st + ((MODE == 0) ? REC + dd : 0);  // step constants
-  constexpr int NQ = (NC + 31) / 32;
-  __shared__ double prev_pose[12], prev_cov[36], M[36], newp[12], rec[21], dpz[12], dc[36];
-  __shared__ int prev_node;
-  __shared__ uint8_t prev_rot;
-  const int lane = threadIdx.x;
-  double pre[NQ];
-  int32_t ps = 0, pt = 0;
-  uint8_t prot = 0;
-  auto load_step = [&](int64_t k) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      const int e = lane + 32 * q;
-      if (e < st) pre[q] = dpose[k * st + e];
-      else if (MODE == 0 && e < st + REC) pre[q] = inv_rec[k * REC + (e - st)];
-      else if (MODE == 0 && e < NC) pre[q] = dcov_p[k * dd + (e - st - REC)];
-    }
-    ps = src[k];
-    pt = dst[k];
-    prot = drot[k];
+// The walk: S_k = A S_{k-1} A^T + Sigma_Delta with A = Ad(Delta^-1) known for
+// every step beforehand, and the poses. An FP64 instruction takes 64 cycles of
+// its warp whether or not the next one waits for it, so a step costs what its
+// longest chain of dependent FMAs takes, and the chains are cut to what has to
+// be sequential. In blocks (r: rotation, t: translation; A = [[R, 0], [K, R]]),
+// with the term order of M_elem and C_elem (pcm_math.cuh) kept,
+//   rr' = (R rr) R^T + Q,   tr' = (K rr + R tr) R^T + Q,
+//   tt' = (K rr + R tr) K^T + (K rt + R tt) R^T + Q,
+// so rr needs only rr, tr only rr and tr, and each block's own loop is seven
+// instructions (three products, three products, the sum with Q): one warp per
+// block, each a chunk of steps behind the one before, which hands it its
+// partial sums (K rr; then K rt and the first three terms of tt') through
+// shared memory. The columns M_rt of the first product are never read. The
+// poses are a chain of their own on another SM.
+// Bound by the latency of a step: seven FP64 instructions (448 cycles alone,
+// about 530 with three warps on the SM's FP64 pipe) and the exchange of the
+// block between its lanes twice; 790 cycles in all. 20,000 steps: 3D 18.0 ->
+// 8.0 ms (before: two warps, 13 instructions and two block barriers a step),
+// 2D 20.5 -> 6.5 ms (one warp).
+constexpr int kScanChunk = 16;  // steps per chunk
+
+template <int DIM>
+struct ScanCov {
+  double cst[4][kScanChunk * ScanRec<DIM>::n];
+  double rr[2][kScanChunk][9];   // K rr
+  double tr[2][kScanChunk][18];  // K rt, then the first three terms of tt'
+  int32_t src[4][kScanChunk], dst[4][kScanChunk];
+};
+template <int DIM>
+struct ScanPose {
+  double dp[2][kScanChunk][Lie<DIM>::stride];
+  int32_t src[2][kScanChunk], dst[2][kScanChunk];
+  uint8_t rot[2][kScanChunk];
+};
+
+__device__ __forceinline__ double shfl_d(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// The covariance block of `role` (0 rr or the whole 2D covariance, 1 tr, 2 tt)
+// over the steps [0, n) of chunk c. Lane 3 i + j < 9 holds entry (i, j) of the
+// block (mirrored where it is symmetric: the entry of the lower triangle),
+// lanes 9-17 the second job that shares its instructions; role 1: entry (i, j)
+// of rt. last: the slot written by the step before.
+template <int DIM, int role>
+__device__ __forceinline__ void scan_chunk(int c, int n, ScanCov<DIM>& s, double* __restrict__ cov,
+                                           double& S, int32_t& last, int lane) {
+  constexpr int d = ScanRec<DIM>::d, dd = d * d, ad = ScanRec<DIM>::ad;
+  const bool second = lane >= 9 && lane < 18;
+  const int e = lane < 18 ? lane % 9 : 0, i = e / 3, j = e % 3;
+  // the products' left rows (R or K, row i) and right rows (row b)
+  const int left = (second && DIM == 3 ? 9 : 0) + 3 * i;
+  const bool tri = !(role == 1 && !second);  // a symmetric result: its lower entry (a, b)
+  const int a = tri ? max(i, j) : i, b = tri ? min(i, j) : j;
+  const int right = (role == 1 && second ? 9 : 0) + 3 * b;
+  const int qi = (role ? 3 : 0) + a, qj = (role == 2 ? 3 : 0) + b;
+  const int q = ad + qi * (qi + 1) / 2 + qj;
+  // the entry's place in the covariance
+  const int row = role == 1 ? (second ? i : 3 + i) : (role ? 3 : 0) + i;
+  const int col = role == 1 ? (second ? 3 + j : j) : (role ? 3 : 0) + j;
+  const bool out = lane < 9 || (role == 1 && second);
+  // step k's operands; those of step k + 1 are read while step k computes
+  struct Step {
+    double l0, l1, l2, r0, r1, r2, Q, m0, c0;
+    int32_t from, to;
   };
-  auto store_step = [&]() {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      const int e = lane + 32 * q;
-      if (e < st) dpz[e] = pre[q];
-      else if (MODE == 0 && e < st + REC) rec[e - st] = pre[q];
-      else if (MODE == 0 && e < NC) dc[e - st - REC] = pre[q];
+  auto load = [&](int k) {
+    const double* cst = s.cst[c & 3] + k * ScanRec<DIM>::n;
+    Step x{cst[left], cst[left + 1], cst[left + 2], cst[right], cst[right + 1], cst[right + 2], cst[q], -0.0, -0.0,
+           s.src[c & 3][k], s.dst[c & 3][k]};
+    // what the products are added to (-0 + x = x)
+    if (role == 1) {
+      const double v = s.rr[c & 1][k][e];
+      x.m0 = second ? -0.0 : v;
     }
+    if (role == 2) {
+      x.m0 = s.tr[c & 1][k][e];
+      x.c0 = s.tr[c & 1][k][9 + 3 * a + b];
+    }
+    return x;
   };
-  // this lane's phase-1 items (e = lane, lane + 32 of [M entries | pose
-  // entries]) and phase-2 entry (ii, jj) of the lower triangle, fixed for
-  // the whole walk
-  constexpr int nm = (MODE == 0) ? dd : 0;
-  int it_i[2], it_k[2], it_pl[2];
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int e = lane + 32 * q;
-    it_i[q] = -1;
-    it_k[q] = 0;
-    it_pl[q] = -1;
-    if (e < nm) {
-      it_i[q] = e / d;
-      it_k[q] = e % d;
-    } else if (e < nm + st) {
-      it_pl[q] = e - nm;
-    }
-  }
-  constexpr int ntri = d * (d + 1) / 2;
-  int tri_i = 0, tri_j = 0;
-  if (lane < ntri) {
-    int idx = lane;
-    while (idx > tri_i) {
-      idx -= tri_i + 1;
-      ++tri_i;
-    }
-    tri_j = idx;
-  }
-  int32_t last_dst = -1;
-  if (count > 0) {
-    load_step(0);
-    store_step();
-  }
-  int32_t s = ps, t = pt;
-  uint8_t rot_k = prot;
-  for (int64_t k = 0; k < count; ++k) {
-    if (k + 1 < count) load_step(k + 1);
-    // load previous state (unless it is the pose just written)
-    if (s != last_dst) {
-      for (int e = lane; e < st; e += 32) prev_pose[e] = tr.pose[(size_t)s * st + e];
-      if (MODE == 0)
-        for (int e = lane; e < dd; e += 32) prev_cov[e] = tr.cov[(size_t)s * dd + e];
-      if (lane == 0) {
-        prev_rot = tr.rot[s];
-        if (MODE == 1) prev_node = tr.node[s];
-      }
-    }
-    __syncwarp();
-    // phase 1: M = Ad(Delta^-1) S_prev (items [0, dd)) and the new pose
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      if (it_i[q] >= 0) {
-        if constexpr (DIM == 3) M[lane + 32 * q] = p3_M_elem(rec, rec + 9, prev_cov, it_i[q], it_k[q]);
-        else M[lane + 32 * q] = p2_M_elem(rec, prev_cov, it_i[q], it_k[q]);
-      } else if (it_pl[q] >= 0) {
-        if constexpr (DIM == 3) newp[it_pl[q]] = p3_compose_elem(prev_pose, dpz, it_pl[q]);
-        else newp[it_pl[q]] = p2_compose_elem(prev_pose, dpz, it_pl[q]);
-      }
-    }
-    __syncwarp();
-    // phase 2: lower triangle of M Ad^T + S_Delta
-    if (MODE == 0) {
-      double v = 0.0;
-      const int ii = tri_i, jj = tri_j;
-      if (lane < ntri) {
-        double c;
-        if constexpr (DIM == 3) c = p3_C_elem(rec, rec + 9, M + 6 * ii, jj);
-        else c = p2_C_elem(rec, M + 3 * ii, jj);
-        v = add(c, dc[d * ii + jj]);
-      }
+  double* const place = cov + d * row + col;
+  Step cur = load(0);
+  bool again = cur.from != last;
+  for (int k = 0; k < n; ++k) {
+    if (again) {  // the chain continues from an older pose: read it back
       __syncwarp();
-      if (lane < ntri) {
-        prev_cov[d * ii + jj] = v;
-        prev_cov[d * jj + ii] = v;
-      }
+      S = out ? place[(size_t)cur.from * dd] : 0.0;
     }
-    for (int e = lane; e < st; e += 32) prev_pose[e] = newp[e];
-    if (lane == 0) {
-      prev_rot = (prev_rot && rot_k) ? 1 : 0;
-      if (MODE == 1) prev_node = prev_node + 1;
+    // M: left row times column j of the block (lanes 9-17 of role 1: of rt)
+    const int at = (role == 1 && second ? 9 : 0) + j;
+    const double s0 = shfl_d(S, at), s1 = shfl_d(S, at + 3), s2 = shfl_d(S, at + 6);
+    double M = fmad(cur.l0, s0, cur.m0);
+    const Step nxt = load(min(k + 1, n - 1));
+    M = fmad(cur.l1, s1, M);
+    M = fmad(cur.l2, s2, M);
+    const double t0 = shfl_d(M, 3 * a), t1 = shfl_d(M, 3 * a + 1), t2 = shfl_d(M, 3 * a + 2);
+    // C: row a of M times the right row
+    double C = fmad(t0, cur.r0, cur.c0);
+    if (second && role == 0 && DIM == 3) s.rr[c & 1][k][e] = M;
+    if (second && role == 1) s.tr[c & 1][k][e] = M;
+    C = fmad(t1, cur.r1, C);
+    C = fmad(t2, cur.r2, C);
+    S = add(C, cur.Q);
+    if (second && role == 1) s.tr[c & 1][k][9 + e] = C;
+    again = nxt.from != cur.to;
+    double* const o = place + (size_t)cur.to * dd;
+    cur = nxt;
+    if (role == 1) {
+      const double x = shfl_d(S, 3 * j + i);  // rt = tr^T
+      if (second) S = x;
     }
-    __syncwarp();
-    for (int e = lane; e < st; e += 32) tr.pose[(size_t)t * st + e] = prev_pose[e];
-    if (MODE == 0)
-      for (int e = lane; e < dd; e += 32) tr.cov[(size_t)t * dd + e] = prev_cov[e];
-    if (lane == 0) {
-      tr.rot[t] = prev_rot;
-      if (MODE == 1) tr.node[t] = prev_node;
-    }
-    last_dst = t;
-    __syncwarp();
-    if (k + 1 < count) {
-      store_step();
-      s = ps;
-      t = pt;
-      rot_k = prot;
-    }
-    __syncwarp();
+    if (out) *o = S;
+  }
+  last = s.dst[c & 3][n - 1];
+}
+
+// chunk c's constants, by one warp (it has the time of a chunk for it: a copy
+// that gathered the record's parts from two arrays took longer than that)
+template <int DIM>
+__device__ __forceinline__ void scan_load(int c, int n, ScanCov<DIM>& s, const int32_t* __restrict__ src,
+                                          const int32_t* __restrict__ dst, const double* __restrict__ rec, int lane) {
+  constexpr int nc = ScanRec<DIM>::n;
+  const int64_t k0 = (int64_t)c * kScanChunk;
+  const double* from = rec + k0 * nc;
+  double* to = s.cst[c & 3];
+#pragma unroll 10
+  for (int x = lane; x < n * nc; x += 32) to[x] = from[x];
+  if (lane < n) {
+    s.src[c & 3][lane] = src[k0 + lane];
+    s.dst[c & 3][lane] = dst[k0 + lane];
   }
 }
 
-// The 3D PoseWithCovariance walk on two warps (64 threads), one output
-// element per thread. Every element of compose (GeometryUtils.h:119-129) is
-// an FMA chain over at most six products, evaluated exactly as p3_M_elem,
-// p3_C_elem and p3_compose_elem do (a chain that starts with a product
-// starts from fma(a0, b0, -0), which equals mul(a0, b0) bit for bit, so the
-// threads run one branch-free chain): warp 0 takes the three-term chains
-// (rows 0-2 of M = Ad(Delta^-1) S, the new pose, the C entries of columns
-// 0-2), warp 1 the six-term chains (rows 3-5 of M, the C entries of columns
-// 3-5), so both warps issue their FP64 chains on their own sub-partitions.
-// Step constants are double-buffered in shared memory: the next step's are
-// loaded while this one computes. Two block barriers per step.
-__global__ void __launch_bounds__(64) k_traj_scan_pwc3(int64_t count, const int32_t* __restrict__ src,
-                                                       const int32_t* __restrict__ dst,
-                                                       const double* __restrict__ dpose,
-                                                       const double* __restrict__ inv_rec,
-                                                       const double* __restrict__ dcov_p,
-                                                       const uint8_t* __restrict__ drot, TrajView tr) {
-  constexpr int st = 12, dd = 36, REC = 21, NC = st + REC + dd;  // 69 step constants
-  __shared__ double prev_pose[12], prev_cov[36], M[36];
-  __shared__ double cst[2][72];  // [0,12) Delta pose, [12,33) Ad(Delta^-1) pieces (R, K, t), [33,69) Sigma_Delta
-  __shared__ uint8_t prev_rot;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // ---- this thread's chains (fixed for the whole walk)
-  // phase 1 kind: 0 none, 1 M row < 3, 2 pose R entry, 3 pose t entry, 4 M row >= 3
-  int p1 = 0, mi = 0, mk = 0, pe = 0;
-  if (warp == 0) {
-    if (lane < 18) {
-      p1 = 1;
-      mi = lane / 6;
-      mk = lane % 6;
-    } else if (lane < 27) {
-      p1 = 2;
-      pe = lane - 18;
-    } else if (lane < 30) {
-      p1 = 3;
-      pe = 9 + (lane - 27);
-    }
-  } else if (lane < 18) {
-    p1 = 4;
-    mi = 3 + lane / 6;
-    mk = lane % 6;
-  }
-  // phase 2: lower-triangle entry (ci, cj) of M Ad^T
-  int p2 = 0, ci = 0, cj = 0;
-  if (warp == 0 && lane < 15) {  // columns 0-2: rows cj..5 of each column
-    int idx = lane;
-    cj = 0;
-    while (idx >= 6 - cj) {
-      idx -= 6 - cj;
-      ++cj;
-    }
-    ci = cj + idx;
-    p2 = 1;
-  } else if (warp == 1 && lane < 6) {  // columns 3-5, rows >= column
-    const int tab_i[6] = {3, 4, 5, 4, 5, 5}, tab_j[6] = {3, 3, 3, 4, 4, 5};
-    ci = tab_i[lane];
-    cj = tab_j[lane];
-    p2 = 2;
-  }
-  double pre[2];
-  int32_t ps = 0, pt = 0;
-  uint8_t prot = 0;
-  auto load_step = [&](int64_t k) {
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int e = tid + 64 * q;
-      if (e < st) pre[q] = dpose[k * st + e];
-      else if (e < st + REC) pre[q] = inv_rec[k * REC + (e - st)];
-      else if (e < NC) pre[q] = dcov_p[k * dd + (e - st - REC)];
-    }
-    ps = src[k];
-    pt = dst[k];
-    prot = drot[k];
-  };
-  auto store_step = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int e = tid + 64 * q;
-      if (e < NC) cst[buf][e] = pre[q];
-    }
-  };
-  int32_t last_dst = -1;
-  if (count > 0) {
-    load_step(0);
-    store_step(0);
-  }
-  __syncthreads();
-  int32_t s = ps, t = pt;
-  uint8_t rot_k = prot;
-  for (int64_t k = 0; k < count; ++k) {
-    const int b = (int)(k & 1);
-    const double* dpz = cst[b];
-    const double* R = cst[b] + 12;
-    const double* K = cst[b] + 21;
-    const double* dc = cst[b] + 33;
-    if (k + 1 < count) load_step(k + 1);
-    if (s != last_dst) {  // the chain continues from an older pose: read it back
-      for (int e = tid; e < st; e += 64) prev_pose[e] = tr.pose[(size_t)s * st + e];
-      for (int e = tid; e < dd; e += 64) prev_cov[e] = tr.cov[(size_t)s * dd + e];
-      if (tid == 0) prev_rot = tr.rot[s];
-      __syncthreads();
-    }
-    // ---- phase 1
-    double newp = 0.0;
-    if (p1 != 0) {
-      double a[6], x[6], c0 = -0.0;
-      int nt = 3;
-      if (p1 == 1) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          a[q] = R[3 * mi + q];
-          x[q] = prev_cov[6 * q + mk];
-        }
-      } else if (p1 == 4) {
-        const int r = mi - 3;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          a[q] = K[3 * r + q];
-          x[q] = prev_cov[6 * q + mk];
-          a[3 + q] = R[3 * r + q];
-          x[3 + q] = prev_cov[18 + 6 * q + mk];
-        }
-        nt = 6;
-      } else if (p1 == 2) {
-        const int i = pe / 3, j = pe % 3;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          a[q] = prev_pose[3 * i + q];
-          x[q] = dpz[3 * q + j];
-        }
-      } else {
-        const int i = pe - 9;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          a[q] = prev_pose[3 * i + q];
-          x[q] = dpz[9 + q];
-        }
-        c0 = prev_pose[9 + i];
-      }
-      double acc = fmad(a[0], x[0], c0);
-      acc = fmad(a[1], x[1], acc);
-      acc = fmad(a[2], x[2], acc);
-      if (nt == 6) {
-        acc = fmad(a[3], x[3], acc);
-        acc = fmad(a[4], x[4], acc);
-        acc = fmad(a[5], x[5], acc);
-      }
-      if (p1 == 1 || p1 == 4) M[6 * mi + mk] = acc;
-      else newp = acc;
-    }
-    __syncthreads();
-    // ---- phase 2: C = M Ad^T + Sigma_Delta (lower triangle, mirrored), the new pose
-    if (p2 != 0) {
-      const double* m = M + 6 * ci;
-      double acc;
-      if (p2 == 1) {
-        acc = fmad(m[0], R[3 * cj], -0.0);
-        acc = fmad(m[1], R[3 * cj + 1], acc);
-        acc = fmad(m[2], R[3 * cj + 2], acc);
-      } else {
-        const double* kk = K + 3 * (cj - 3);
-        const double* rr = R + 3 * (cj - 3);
-        acc = fmad(m[0], kk[0], -0.0);
-        acc = fmad(m[1], kk[1], acc);
-        acc = fmad(m[2], kk[2], acc);
-        acc = fmad(m[3], rr[0], acc);
-        acc = fmad(m[4], rr[1], acc);
-        acc = fmad(m[5], rr[2], acc);
-      }
-      const double v = add(acc, dc[6 * ci + cj]);
-      prev_cov[6 * ci + cj] = v;
-      prev_cov[6 * cj + ci] = v;
-      tr.cov[(size_t)t * dd + 6 * ci + cj] = v;
-      if (ci != cj) tr.cov[(size_t)t * dd + 6 * cj + ci] = v;
-    }
-    if (p1 == 2 || p1 == 3) {
-      prev_pose[pe] = newp;
-      tr.pose[(size_t)t * st + pe] = newp;
-    }
-    if (tid == 0) {
-      prev_rot = (prev_rot && rot_k) ? 1 : 0;
-      tr.rot[t] = prev_rot;
-    }
-    last_dst = t;
-    if (k + 1 < count) {
-      store_step(b ^ 1);
-      s = ps;
-      t = pt;
-      rot_k = prot;
+template <int DIM>
+__device__ void scan_cov(int64_t count, const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
+                         const double* __restrict__ rec, TrajView tr, ScanCov<DIM>& s) {
+  constexpr int roles = DIM == 3 ? 3 : 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunks = (int)((count + kScanChunk - 1) / kScanChunk);
+  double S = 0.0;
+  int32_t last = -1;
+  // warp w < roles works on chunk it - 1 - w, the last warp loads chunk it
+  for (int it = 0; it < chunks + roles; ++it) {
+    const int c = warp < roles ? it - 1 - warp : it;
+    if (c >= 0 && c < chunks) {
+      const int n = (int)min((int64_t)kScanChunk, count - (int64_t)c * kScanChunk);
+      if (warp == 0) scan_chunk<DIM, 0>(c, n, s, tr.cov, S, last, lane);
+      else if (DIM == 3 && warp == 1) scan_chunk<DIM, DIM == 3 ? 1 : 0>(c, n, s, tr.cov, S, last, lane);
+      else if (DIM == 3 && warp == 2) scan_chunk<DIM, DIM == 3 ? 2 : 0>(c, n, s, tr.cov, S, last, lane);
+      else if (warp == 3) scan_load<DIM>(c, n, s, src, dst, rec, lane);
     }
     __syncthreads();
   }
+}
+
+// The poses (and node counts): lane e computes entry e of the new pose, the
+// operations of p3_compose / p2_compose (one instruction stream for all
+// entries: diverging lanes would issue theirs one after another).
+template <int DIM, int MODE>
+__device__ void scan_pose(int64_t count, const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
+                          const double* __restrict__ dpose, const uint8_t* __restrict__ drot, TrajView tr,
+                          ScanPose<DIM>& s) {
+  constexpr int st = Lie<DIM>::stride;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunks = (int)((count + kScanChunk - 1) / kScanChunk);
+  double P = 0.0;
+  int32_t last = -1, node = 0;
+  uint8_t rot = 0;
+  const int e = lane < st ? lane : 0;
+  const int i = e < 9 ? e / 3 : e - 9, j = e < 9 ? e % 3 : 0;
+  for (int it = 0; it <= chunks; ++it) {
+    const int c = warp == 0 ? it - 1 : it;
+    const int64_t k0 = (int64_t)c * kScanChunk;
+    const int n = c >= 0 && c < chunks ? (int)min((int64_t)kScanChunk, count - k0) : 0;
+    if (warp == 3) {
+      for (int x = lane; x < n * st; x += 32) s.dp[c & 1][x / st][x % st] = dpose[k0 * st + x];
+      if (lane < n) {
+        s.src[c & 1][lane] = src[k0 + lane];
+        s.dst[c & 1][lane] = dst[k0 + lane];
+        s.rot[c & 1][lane] = drot[k0 + lane];
+      }
+    } else if (warp == 0) {
+      for (int k = 0; k < n; ++k) {
+        const double* D = s.dp[c & 1][k];
+        const int32_t from = s.src[c & 1][k], to = s.dst[c & 1][k];
+        if (from != last) {  // the chain continues from an older pose: read it back
+          __syncwarp();
+          P = tr.pose[(size_t)from * st + e];
+          rot = tr.rot[from];
+          if (MODE == 1) node = tr.node[from];
+        }
+        if constexpr (DIM == 3) {
+          const bool t = e >= 9;
+          const double x0 = t ? D[9] : D[j], x1 = t ? D[10] : D[3 + j], x2 = t ? D[11] : D[6 + j];
+          double acc = fmad(shfl_d(P, 3 * i), x0, t ? P : -0.0);
+          acc = fmad(shfl_d(P, 3 * i + 1), x1, acc);
+          P = fmad(shfl_d(P, 3 * i + 2), x2, acc);
+        } else {
+          // (c, s, x, y): u and w are the two products of the entry's formula
+          const double ac = shfl_d(P, 0), as = shfl_d(P, 1);
+          const double u = mul(e & 1 ? ac : as, e < 2 ? D[1] : D[3]);
+          const double w = fmad(e & 1 ? as : ac, e < 2 ? D[0] : D[2], e & 1 ? u : -u);
+          const double x = add(P, w);
+          P = e < 2 ? w : x;
+        }
+        rot = rot && s.rot[c & 1][k] ? 1 : 0;
+        ++node;
+        if (lane < st) tr.pose[(size_t)to * st + lane] = P;
+        if (lane == 0) {
+          tr.rot[to] = rot;
+          if (MODE == 1) tr.node[to] = node;
+        }
+        last = to;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// block 0: the covariances (MODE 0), the other one: the poses
+template <int DIM, int MODE>
+__global__ void __launch_bounds__(128) k_traj_scan(int64_t count, const int32_t* __restrict__ src,
+                                                   const int32_t* __restrict__ dst,
+                                                   const double* __restrict__ dpose,
+                                                   const double* __restrict__ rec,
+                                                   const uint8_t* __restrict__ drot, TrajView tr) {
+  __shared__ __align__(8) unsigned char raw[sizeof(ScanCov<DIM>) > sizeof(ScanPose<DIM>) ? sizeof(ScanCov<DIM>)
+                                                                                       : sizeof(ScanPose<DIM>)];
+  if (MODE == 0 && blockIdx.x == 0)
+    scan_cov<DIM>(count, src, dst, rec, tr, *reinterpret_cast<ScanCov<DIM>*>(raw));
+  else
+    scan_pose<DIM, MODE>(count, src, dst, dpose, drot, tr, *reinterpret_cast<ScanPose<DIM>*>(raw));
 }
 
 // ------------------------------------------------------------------ K1
@@ -902,28 +780,26 @@ __global__ void k_symmetrize(int n, int row_begin, const uint32_t* __restrict__ 
 // ------------------------------------------------------------------ launchers
 void launch_traj_scan(int dim, int mode, int64_t count, const int32_t* src, const int32_t* dst,
                       const double* dpose, const double* dcov, TrajView tr, DeviceBuffer<double>& scratch_rec,
-                      DeviceBuffer<double>& scratch_cov, DeviceBuffer<uint8_t>& scratch_rot, cudaStream_t st) {
+                      DeviceBuffer<uint8_t>& scratch_rot, cudaStream_t st) {
   if (count <= 0) return;
-  const int d = dim == 3 ? 6 : 3;
-  scratch_rec.resize((size_t)count * (dim == 3 ? 21 : 9));
-  scratch_cov.resize((size_t)count * d * d);
+  scratch_rec.resize((size_t)count * (dim == 3 ? ScanRec<3>::n : ScanRec<2>::n));
   scratch_rot.resize((size_t)count);
   const int tb = 128;
-  if (dim == 3) k_odom_prep<3><<<div_up(count, tb), tb, 0, st>>>(count, dpose, dcov, scratch_rec.get(),
-                                                                   scratch_cov.get(), scratch_rot.get());
-  else k_odom_prep<2><<<div_up(count, tb), tb, 0, st>>>(count, dpose, dcov, scratch_rec.get(), scratch_cov.get(),
-                                                        scratch_rot.get());
+  if (dim == 3)
+    k_odom_prep<3><<<div_up(count, tb), tb, 0, st>>>(count, dpose, dcov, scratch_rec.get(), scratch_rot.get());
+  else
+    k_odom_prep<2><<<div_up(count, tb), tb, 0, st>>>(count, dpose, dcov, scratch_rec.get(), scratch_rot.get());
   RPGO_LAUNCHED();
+  const int blocks = mode == 0 ? 2 : 1;
+  auto scan = [&](auto kernel) {
+    kernel<<<blocks, 128, 0, st>>>(count, src, dst, dpose, scratch_rec.get(), scratch_rot.get(), tr);
+  };
   if (dim == 3) {
-    if (mode == 0) k_traj_scan_pwc3<<<1, 64, 0, st>>>(count, src, dst, dpose, scratch_rec.get(), scratch_cov.get(),
-                                                     scratch_rot.get(), tr);
-    else k_traj_scan<3, 1><<<1, 32, 0, st>>>(count, src, dst, dpose, scratch_rec.get(), scratch_cov.get(),
-                                             scratch_rot.get(), tr);
+    if (mode == 0) scan(k_traj_scan<3, 0>);
+    else scan(k_traj_scan<3, 1>);
   } else {
-    if (mode == 0) k_traj_scan<2, 0><<<1, 32, 0, st>>>(count, src, dst, dpose, scratch_rec.get(), scratch_cov.get(),
-                                                       scratch_rot.get(), tr);
-    else k_traj_scan<2, 1><<<1, 32, 0, st>>>(count, src, dst, dpose, scratch_rec.get(), scratch_cov.get(),
-                                             scratch_rot.get(), tr);
+    if (mode == 0) scan(k_traj_scan<2, 0>);
+    else scan(k_traj_scan<2, 1>);
   }
   RPGO_LAUNCHED();
 }

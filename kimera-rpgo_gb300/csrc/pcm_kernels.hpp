@@ -20,7 +20,7 @@ struct TrajView {
 // mode 0: PoseWithCovariance (Pcm), 1: PoseWithNode (PcmSimple)
 void launch_traj_scan(int dim, int mode, int64_t count, const int32_t* src, const int32_t* dst,
                       const double* dpose, const double* dcov, TrajView tr, DeviceBuffer<double>& scratch_rec,
-                      DeviceBuffer<double>& scratch_cov, DeviceBuffer<uint8_t>& scratch_rot, cudaStream_t st);
+                      DeviceBuffer<uint8_t>& scratch_rot, cudaStream_t st);
 
 void launch_odom_check(int dim, int mode, int64_t count, const int32_t* si, const int32_t* sj, const double* zp,
                        const double* zc, TrajView tr, double th0, double th1, uint8_t* ok, cudaStream_t st);
