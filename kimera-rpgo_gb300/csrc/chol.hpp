@@ -28,7 +28,7 @@ struct CholDev {
   DeviceBuffer<double> out;   // model change, status
   DeviceBuffer<double> Hs;    // H in the block layout of L (per linearisation)
   DeviceBuffer<double> dampS; // damping diagonal of the diagonal blocks, same layout
-  DeviceBuffer<int32_t> status;  // pivot failure; a wait of the dataflow part ran out
+  DeviceBuffer<int32_t> status;  // pivot failure; a wait of the dataflow part ran out; CTAs done
   // dataflow part (chol_plan.hpp) and the words its columns hand on: update
   // products, forward and backward solutions
   DeviceBuffer<int32_t> df_col, df_blk, df_dst, df_pre, df_row, df_trow;

@@ -85,7 +85,7 @@ struct CholArgs {
   size_t df_prod_n;
   const int32_t *df_col, *df_blk, *df_dst, *df_pre, *df_row, *df_trow;
   double *prod, *ys, *xs;
-  int32_t* df_stall;
+  int32_t *df_stall, *ticket;
 };
 
 // end of level l's tasks and columns (the compacted lists of a joint batch
@@ -1041,6 +1041,7 @@ __device__ void tail_backward_item(const CholArgs& a, double* yt, int k, TileSme
 // 780.
 constexpr unsigned long long kEmpty = 0x7ffcd5c3a19b42e7ull;  // a NaN that no operation produces
 constexpr int kDfSpins = 1 << 21;
+constexpr int kPivotBar = 3;           // named barriers 3 .. 3 + D - 1: a column of L_jj is in place
 constexpr int kDfMat = kThreads - 32;  // warps 0-6: the column's blocks; warp 7: its right-hand side
 
 __device__ __forceinline__ double ld_word(const double* p) {
@@ -1054,23 +1055,45 @@ __device__ __forceinline__ void st_word(double* p, double v) {
 __device__ __forceinline__ bool is_empty(double v) {
   return (unsigned long long)__double_as_longlong(v) == kEmpty;
 }
+// one more poll of a wait found nothing; true (in all lanes of the warp) when
+// the wait has to end
+__device__ __forceinline__ bool df_give_up(const CholArgs& a, int& spins) {
+  if ((++spins & 1023) != 0) return false;
+  if (spins >= kDfSpins) atomicExch(a.df_stall, 1);
+  return __any_sync(kFull, *(volatile int32_t*)a.df_stall != 0);
+}
 // Words p[0], p[step], ... (n <= N of them, 0 in lanes without) as soon as
 // every lane of the warp has its own; all lanes of the warp call it.
 template <int N>
 __device__ __forceinline__ void ld_words(const CholArgs& a, const double* p, int step, int n, double (&v)[N]) {
   int spins = 0;
-  while (true) {
+  do {
     bool all = true;
 #pragma unroll
     for (int k = 0; k < N; ++k) v[k] = k < n ? ld_word(p + (size_t)k * step) : 0.0;
 #pragma unroll
     for (int k = 0; k < N; ++k) all = all && !is_empty(v[k]);
     if (__all_sync(kFull, all)) return;
-    if ((++spins & 1023) == 0) {
-      if (spins >= kDfSpins) atomicExch(a.df_stall, 1);
-      if (__any_sync(kFull, *(volatile int32_t*)a.df_stall != 0)) return;
+  } while (!df_give_up(a, spins));
+}
+// v (+)= words 0 .. n - 1 of a window of N (p, step as above), added in that
+// order; every G words are a partial sum of their own (a chunk), added to v
+// when it is complete. first: v has no value yet. (Adding each word as it
+// arrives, with a vote per word, made a solve 5 to 15 % slower.)
+template <int N, int G>
+__device__ __forceinline__ void add_words(const CholArgs& a, const double* p, int step, int n, bool first,
+                                          double& v) {
+  double x[N];
+  ld_words<N>(a, p, step, n, x);
+#pragma unroll
+  for (int h = 0; h < N; h += G)
+    if (h < n) {
+      double tot = x[h];
+#pragma unroll
+      for (int k = 1; k < G; ++k)
+        if (h + k < n) tot += x[h + k];
+      v = first && h == 0 ? tot : v + tot;
     }
-  }
 }
 
 __device__ __forceinline__ bool df_on(const CholArgs& a, int j) {
@@ -1096,7 +1119,8 @@ __device__ __forceinline__ bool positive(double v) {
 // Cholesky of S_jj by one warp, one lane per entry of the lower part: each
 // pivot costs a reciprocal square root, one product and one FMA on the FP64
 // pipe (64 cycles each whatever the lanes do), where a lane per row issues an
-// FMA per column. The same operations per entry as factor_diag.
+// FMA per column. The same operations per entry as factor_diag. Each column of
+// L_jj is published as soon as it is scaled.
 template <int D>
 __device__ __forceinline__ void df_factor(const CholArgs& a, int j, int lane, DfSmem<D>& s) {
   constexpr int ntri = D * (D + 1) / 2;
@@ -1110,7 +1134,11 @@ __device__ __forceinline__ void df_factor(const CholArgs& a, int j, int lane, Df
     const bool pos = positive(piv);
     ok = ok && pos;
     const double il = rsqrt(pos ? piv : 1.0);
-    if (c == k) v = r == k ? il : v * il;
+    if (c == k) {
+      v = r == k ? il : v * il;
+      if (lane < ntri) s.Lj[r * D + c] = v;
+    }
+    asm volatile("bar.arrive %0, %1;" ::"r"(kPivotBar + k), "n"(kDfMat) : "memory");
     if (k + 1 < D) {
       const double lr = __shfl_sync(kFull, v, r >= k ? r * (r + 1) / 2 + k : 0);
       const double lc = __shfl_sync(kFull, v, c >= k ? c * (c + 1) / 2 + k : 0);
@@ -1118,10 +1146,7 @@ __device__ __forceinline__ void df_factor(const CholArgs& a, int j, int lane, Df
     }
   }
   if (!ok && lane == 0) set_fail(sys_status(a, j));
-  if (lane < ntri) {
-    s.Lj[r * D + c] = v;
-    a.Ldiag[(size_t)j * D * D + r * D + c] = v;
-  }
+  if (lane < ntri) a.Ldiag[(size_t)j * D * D + r * D + c] = v;
 }
 
 // Row r of a forward row sum over n entries of df_row from `row` on, by one
@@ -1192,43 +1217,36 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
       double v = (on && bl.y == 0) ? block_H<D>(a, p0 + b, b == 0, e / D, e % D) : 0.0;
       constexpr int W = D == 6 ? 2 * G : G;  // words per wait
       const int n = __reduce_max_sync(kFull, bl.y);
-      for (int u = 0; u < n; u += W) {
-        double x[W];
-        ld_words<W>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, x);
-#pragma unroll
-        for (int h = 0; h < W; h += G)
-          if (u + h < bl.y) {
-            double tot = x[h];
-#pragma unroll
-            for (int k = 1; k < G; ++k)
-              if (u + h + k < bl.y) tot += x[h + k];
-            v = u + h == 0 ? tot : v + tot;
-          }
-      }
+      for (int u = 0; u < n; u += W)
+        add_words<W, G>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, u == 0, v);
       __syncwarp();
       if (on) s.S[it] = v;
     }
     df_mat_sync();
+    // Warp 0 factors S_jj; the others solve L_ij = S_ij L_jj^-T behind it, one
+    // row per lane group and one entry per lane (solve_offdiag's operations),
+    // a pivot as soon as warp 0 has published its column of L_jj (named barrier
+    // kPivotBar + pivot: warp 0 arrives, the others wait), so that little of
+    // the solve is left after the last pivot.
     if (wi == 0) {
       df_factor<D>(a, j, lane, s);
       asm volatile("bar.arrive 2, 64;" ::: "memory");  // L_jj for the right-hand side's warp
-    }
-    df_mat_sync();
-    // L_ij = S_ij L_jj^-T, one row per lane group, one entry per lane
-    // (solve_offdiag's operations)
-    for (int rr0 = wi * G; rr0 < m * D; rr0 += kDfMat / 32 * G) {
-      const int rr = rr0 + g;
-      const bool on = g < G && rr < m * D;
-      double v = on ? s.S[dd + rr * D + r] : 0.0;
+    } else {
+      for (int rr0 = 0; rr0 == 0 || rr0 < m * D; rr0 += (kDfMat / 32 - 1) * G) {
+        const int rr = rr0 + (wi - 1) * G + g;
+        const bool on = g < G && rr < m * D;
+        double v = on ? s.S[dd + rr * D + r] : 0.0;
 #pragma unroll
-      for (int c = 0; c < D; ++c) {
-        const double x = __shfl_sync(kFull, v, base + c) * s.Lj[c * D + c];
-        if (r == c) v = x;
-        else if (r > c) v = fma(-x, s.Lj[r * D + c], v);
-      }
-      if (on) {
-        s.S[dd + rr * D + r] = v;
-        st_word(a.L + (size_t)(p0 + 1) * dd + rr * D + r, v);
+        for (int c = 0; c < D; ++c) {
+          if (rr0 == 0) asm volatile("bar.sync %0, %1;" ::"r"(kPivotBar + c), "n"(kDfMat) : "memory");
+          const double x = __shfl_sync(kFull, v, base + c) * s.Lj[c * D + c];
+          if (r == c) v = x;
+          else if (r > c) v = fma(-x, s.Lj[r * D + c], v);
+        }
+        if (on) {
+          s.S[dd + rr * D + r] = v;
+          st_word(a.L + (size_t)(p0 + 1) * dd + rr * D + r, v);
+        }
       }
     }
     df_mat_sync();
@@ -1275,6 +1293,7 @@ template <int D>
 __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
   constexpr int dd = D * D;
   const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31, n = a.T * D;
+  if (n == 0) return;
   double* yt = a.y + (size_t)a.ns * D;
   double b = 0.0;  // warp 7: the right-hand side, a row per lane
   if (wi < kDfMat / 32) {
@@ -1291,44 +1310,57 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
                      : gather_offdiag<D>(a.fH64, a.ta_src, a.ta_ptr[t], a.ta_ptr[t + 1], rr, cc);
       constexpr int W = 8;
       const int np = __reduce_max_sync(kFull, bl.y);
-      for (int u = 0; u < np; u += W) {
-        double x[W];
-        ld_words<W>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, x);
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-          if (u + k < bl.y) v += x[k];
-      }
+      for (int u = 0; u < np; u += W)
+        add_words<W, 1>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, false, v);
       __syncwarp();
       if (on) s.X[bi * D + rr][bj * D + cc] = v;
     }
     df_mat_sync();
-    for (int c = 0; c < n; ++c) {
-      // warp 0 takes the pivot and scales the column, all update the rest
-      if (wi == 0) {
-        const double piv = s.X[c][c];
+    // Right-looking, one column per step: warp 0 (a row per lane) scales
+    // column c and brings column c + 1 up to date by itself, so that its next
+    // pivot does not wait for the block; the other warps subtract column c
+    // from the columns behind, an entry per thread.
+    constexpr int kOthers = kDfMat - 32;
+    int er[2], eq[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      int e = (int)threadIdx.x - 32 + x * kOthers;
+      er[x] = eq[x] = 0;
+      if (wi > 0 && e < n * (n + 1) / 2) {
+        while (e > er[x]) e -= ++er[x];
+        eq[x] = e;
+      }
+    }
+    // Named barriers: 3 publishes column c (warp 0 arrives, the others wait),
+    // 4 and 5 in turn say that the others are done with it (they arrive, warp 0
+    // waits one step later; it arrives at 3 for column c + 1 before that, so the
+    // others can be one step ahead of its wait, and no more).
+    auto wait = [](int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDfMat) : "memory"); };
+    auto arrive = [](int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kDfMat) : "memory"); };
+    if (wi == 0) {
+      double col = lane < n ? s.X[lane][0] : 0.0;
+      for (int c = 0; c < n; ++c) {
+        const double piv = __shfl_sync(kFull, col, c);
         const bool pos = positive(piv);
-        const int row = c + 1 + lane;
-        const double x = row < n ? s.X[row][c] : 0.0;
         const double il = rsqrt(pos ? piv : 1.0);
-        if (row < n) s.X[row][c] = x * il;
-        __syncwarp();
-        if (lane == 0) {
-          if (!pos) set_fail(a.status);
-          s.X[c][c] = il;
-        }
+        if (!pos && lane == 0) set_fail(a.status);
+        const double l = lane == c ? il : col * il;
+        if (lane >= c && lane < n) s.X[lane][c] = l;
+        arrive(3);
+        if (c > 0) wait(4 + ((c - 1) & 1));
+        // column c + 1: the others have subtracted columns 0 .. c - 1 from it
+        const double lq = __shfl_sync(kFull, l, min(c + 1, n - 1));
+        if (lane > c && lane < n && c + 1 < n) col = fma(-l, lq, s.X[lane][c + 1]);
       }
-      df_mat_sync();
-      const int mr = n - c - 1;
-      for (int e = threadIdx.x; e < mr * (mr + 1) / 2; e += kDfMat) {
-        // entry e of the lower triangle, row by row
-        int r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
-        while (r * (r + 1) / 2 > e) --r;
-        while ((r + 1) * (r + 2) / 2 <= e) ++r;
-        const int q = c + 1 + e - r * (r + 1) / 2;
-        r += c + 1;
-        s.X[r][q] = fma(-s.X[r][c], s.X[q][c], s.X[r][q]);
+      wait(4 + ((n - 1) & 1));
+    } else {
+      for (int c = 0; c < n; ++c) {
+        wait(3);
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          if (eq[x] > c + 1) s.X[er[x]][eq[x]] = fma(-s.X[er[x]][c], s.X[eq[x]][c], s.X[er[x]][eq[x]]);
+        arrive(4 + (c & 1));
       }
-      df_mat_sync();
     }
   } else {
     for (int t = 0; t < a.T; ++t) {
@@ -1338,18 +1370,26 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
   }
   __syncthreads();
   if (wi == kDfMat / 32) {
-    double v = 0.0;
-    for (int c = 0; c < n; ++c) {
-      if (lane == c) v = b * s.X[c][c];
-      const double yc = __shfl_sync(kFull, v, c);
-      if (lane > c && lane < n) b = fma(-s.X[lane][c], yc, b);
-    }
+    double v = 0.0, l[kTB];
+#pragma unroll
+    for (int c = 0; c < kTB; ++c) l[c] = c <= lane && lane < n ? s.X[lane][c] : 0.0;
+#pragma unroll
+    for (int c = 0; c < kTB; ++c)
+      if (c < n) {
+        if (lane == c) v = b * l[c];
+        const double yc = __shfl_sync(kFull, v, c);
+        if (lane > c && lane < n) b = fma(-l[c], yc, b);
+      }
     b = v;
-    for (int c = n - 1; c >= 0; --c) {
-      if (lane == c) v = b * s.X[c][c];
-      const double xc = __shfl_sync(kFull, v, c);
-      if (lane < c) b = fma(-s.X[c][lane], xc, b);
-    }
+#pragma unroll
+    for (int c = 0; c < kTB; ++c) l[c] = c >= lane && c < n ? s.X[c][lane] : 0.0;
+#pragma unroll
+    for (int c = kTB - 1; c >= 0; --c)
+      if (c < n) {
+        if (lane == c) v = b * l[c];
+        const double xc = __shfl_sync(kFull, v, c);
+        if (lane < c) b = fma(-l[c], xc, b);
+      }
     if (lane < n) {
       yt[lane] = v;
       st_word(a.xs + (size_t)a.ns * D + lane, v);
@@ -1451,15 +1491,24 @@ __device__ void df_backward(const CholArgs& a, int lane) {
   }
 }
 
-__device__ __forceinline__ double cta_sum(double v, double* sh) {
+// both sums over the CTA: sum w in lane w < 2 of warp 0 (the other warps would
+// only take turns on the SM's FP64 pipe with it)
+__device__ __forceinline__ double cta_sum2(double v, double w, double (*sh)[2]) {
 #pragma unroll
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[w] = v;
+  for (int o = 16; o; o >>= 1) {
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+    w += __shfl_xor_sync(0xffffffffu, w, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sh[threadIdx.x >> 5][0] = v;
+    sh[threadIdx.x >> 5][1] = w;
+  }
   __syncthreads();
   double t = 0.0;
-  for (int i = 0; i < nw; ++i) t += sh[i];
+  if (threadIdx.x < 2) {
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) t += sh[i][threadIdx.x];
+  }
   return t;
 }
 
@@ -1470,7 +1519,7 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
   __shared__ __align__(16) unsigned char smem[sizeof(TileSmem) > sizeof(DfSmem<D>) ? sizeof(TileSmem)
                                                                                   : sizeof(DfSmem<D>)];
   TileSmem& sm = *reinterpret_cast<TileSmem*>(smem);
-  __shared__ double shr[kThreads / 32];
+  __shared__ double shr[kWarps][2];
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   // Warp-sized work items (tasks, columns) go round-robin over the CTAs, so
@@ -1484,7 +1533,7 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
   double* yt = a.y + (size_t)a.ns * D;
 
   // 1. init
-  if (gt == 0) *a.status = *a.df_stall = 0;
+  if (gt == 0) *a.status = *a.df_stall = *a.ticket = 0;
   if (a.df_cols > 0) df_reset<D>(a, gt, gs);
   for (int k = gt; k < a.G; k += gs) a.b_status[k] = 0;
   for (int k = gt; k < n; k += gs) {
@@ -1703,18 +1752,28 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
     gd = fma(a.g[vi], x, gd);
     dq = fma(a.dampD[vi] * x, x, dq);
   }
-  gd = cta_sum(gd, shr);
-  dq = cta_sum(dq, shr);
-  if (threadIdx.x == 0) {
-    a.part[2 * blockIdx.x] = gd;
-    a.part[2 * blockIdx.x + 1] = dq;
+  // CTAs without an element have nothing to add (and are the last ones); of the
+  // others the one that finishes last adds the sums, in CTA order
+  const int nb = min((int)gridDim.x, (n + kThreads - 1) / kThreads);
+  if ((int)blockIdx.x >= nb) return;
+  const double sum = cta_sum2(gd, dq, shr);
+  __shared__ bool last;
+  if (threadIdx.x < 2) {
+    a.part[2 * blockIdx.x + threadIdx.x] = sum;
+    __threadfence();
   }
-  grid.sync();
-  if (blockIdx.x == 0 && threadIdx.x < 32) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(a.ticket, 1) == nb - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (last && threadIdx.x < 32) {
     double sg = 0.0, sq = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) {
-      sg += a.part[2 * b];
-      sq += a.part[2 * b + 1];
+    for (int b = threadIdx.x; b < nb; b += 32) {
+      sg += __ldcg(a.part + 2 * b);
+      sq += __ldcg(a.part + 2 * b + 1);
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -1892,7 +1951,7 @@ void CholDev::upload(CholPlan&& p, cudaStream_t st) {
   Ldd.resize(std::max<size_t>(1, (size_t)plan.n_tiles * kTB * kTB));
   y.resize((size_t)plan.n_sparse * plan.d + ntp + 1);
   out.resize(4);
-  status.resize(2);
+  status.resize(3);
   df_col.upload(plan.df_col, st);
   df_blk.upload(plan.df_blk, st);
   df_dst.upload(plan.df_dst, st);
@@ -1990,6 +2049,7 @@ static CholArgs make_args(SolverDev& s, CholDev& c, double lambda) {
   a.ys = c.ys.get();
   a.xs = c.xs.get();
   a.df_stall = c.status.get() + 1;
+  a.ticket = c.status.get() + 2;
   return a;
 }
 
