@@ -14,6 +14,7 @@ namespace rpgo {
 struct CholDev {
   CholPlan plan;
   int levels = 0;
+  DeviceBuffer<int32_t> diag_blk;  // per variable: its diagonal block of L, -1 in the dense tail
   DeviceBuffer<int32_t> perm, col_ptr, blk_row, blk_col, lvl_col_ptr, lvl_cols, lvl_task_ptr, tasks, btask, ftask;
   DeviceBuffer<int32_t> upd_ptr, upd_src, tupd_ptr, tupd_src, a_ptr, a_src, ta_ptr, ta_src;
   DeviceBuffer<int32_t> row_ptr, row_blk, trow_ptr, trow_blk, ttasks, ttask_ptr;
@@ -25,7 +26,7 @@ struct CholDev {
   DeviceBuffer<double> part;  // per-CTA partial sums
   DeviceBuffer<double> Spart; // level-task partial sums (D x D per task)
   DeviceBuffer<double> Tpart; // tail row task sums (D per task)
-  DeviceBuffer<double> out;   // model change, status
+  DeviceBuffer<double> out;   // model change, status (chol_solve)
   DeviceBuffer<double> Hs;    // H in the block layout of L (per linearisation)
   DeviceBuffer<double> dampS; // damping diagonal of the diagonal blocks, same layout
   DeviceBuffer<int32_t> status;  // pivot failure; a wait of the dataflow part ran out; CTAs done
@@ -42,15 +43,16 @@ struct CholDev {
 // part takes
 int chol_grid(const SolverDev& s);
 int chol_dataflow_cols(const SolverDev& s);
-// H and the damping diagonal in the block layout of L, from the linearised
-// system (Hd64, fH64, dampD); enqueued after every linearisation.
+// Assembles the linearised system (fH64, fg): the diagonal blocks, the
+// gradient and the damping diagonal per variable, and H and the damping
+// diagonal in the block layout of L; enqueued after every linearisation.
 // mask: a joint batch's variable control words (bit 0: graph in this round)
-void chol_block_hessian(SolverDev& s, CholDev& c, cudaStream_t st, const uint8_t* mask = nullptr);
+void chol_assemble(SolverDev& s, CholDev& c, bool diagonal_damping, cudaStream_t st, const uint8_t* mask = nullptr);
 // Solve with the factorisation of (H + lambda D); fills s.delta.
 SolveOut chol_solve(SolverDev& s, CholDev& c, double lambda, cudaStream_t st);
-// Enqueue the same solve without waiting: the model change and the status
-// are copied to host[0] and host[1] (page-locked) by the stream; call
-// chol_finish after the stream reached that point.
+// Enqueue the same solve without waiting: the kernel writes the model change
+// and the status to host[0] and host[1] (page-locked); call chol_finish after
+// the stream reached that point.
 void chol_enqueue(SolverDev& s, CholDev& c, double lambda, cudaStream_t st, double* host);
 SolveOut chol_finish(SolverDev& s, CholDev& c, const double* host);
 // throws when a solve's status word (0 solved, 1 a failed pivot, 2 a wait

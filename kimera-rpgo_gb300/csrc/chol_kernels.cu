@@ -8,7 +8,7 @@
 //  1. init: right-hand side in elimination order, padding of the dense tail;
 //  2. per elimination-tree level of the sparse columns (leaves first):
 //     (A) the level's tasks over all warps: for every block, its Hessian
-//         block (read from the block layout Hs that k_block_hessian writes
+//         block (read from the block layout Hs that k_assemble_hessian writes
 //         once per linearisation) minus chunks of its L(i,k) L(j,k)^T
 //         updates, and chunks of every column's forward-substitution row
 //         sum; the leaves have no tasks;
@@ -1788,42 +1788,71 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
   }
 }
 
-// H (and the damping diagonal, on diagonal blocks) in the factor's block
-// layout, once per linearisation: thread per block row; an off-diagonal
-// block sums its factors' blocks in the plan's order (each entry the same
+// The assembly, in one launch (it took two, and the second one read back what
+// the first had just written: 16 -> 9 us at 300 poses). The first var_blocks
+// blocks take a warp per variable: lane e owns entries e and e + 32 of its
+// diagonal block (and gradient entry e < D), summed over its factors in their
+// order; written per variable and, with the damping diagonal, in the factor's
+// block layout. The others take a thread per row of an off-diagonal block,
+// which sums its factors' blocks in the plan's order (each entry the same
 // additions as gather_offdiag).
 template <int D>
-__global__ void k_block_hessian(int nblk, const int32_t* __restrict__ blk_row, const int32_t* __restrict__ blk_col,
-                                const int32_t* __restrict__ perm, const int32_t* __restrict__ a_ptr,
-                                const int32_t* __restrict__ a_src, const double* __restrict__ Hd64,
-                                const double* __restrict__ fH64, const double* __restrict__ dampD,
-                                double* __restrict__ Hs, double* __restrict__ dampS,
-                                const uint8_t* __restrict__ mask) {
+__global__ void k_assemble_hessian(int N, int var_blocks, int nblk, const int32_t* __restrict__ inc_ptr,
+                                   const int32_t* __restrict__ inc_fac, const int8_t* __restrict__ inc_role,
+                                   const double* __restrict__ fH64, const double* __restrict__ fg,
+                                   double* __restrict__ Hd64, double* __restrict__ g, double* __restrict__ dampD,
+                                   int diag_damping, const int32_t* __restrict__ diag_blk,
+                                   const int32_t* __restrict__ blk_row, const int32_t* __restrict__ blk_col,
+                                   const int32_t* __restrict__ a_ptr, const int32_t* __restrict__ a_src,
+                                   double* __restrict__ Hs, double* __restrict__ dampS,
+                                   const uint8_t* __restrict__ mask) {
   constexpr int dd = D * D;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if ((int)blockIdx.x < var_blocks) {
+    const int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (v >= N || (mask && !(mask[v] & 1))) return;
+    const int e0 = lane, e1 = lane + 32;
+    double h0 = 0.0, h1 = 0.0, gv = 0.0;
+    for (int k = inc_ptr[v]; k < inc_ptr[v + 1]; ++k) {
+      const int f = inc_fac[k];
+      const int role = inc_role[k];
+      const double* blk = fH64 + (size_t)f * 3 * dd + (role == 1 ? dd : 0);
+      if (e0 < dd) h0 += blk[e0];
+      if (e1 < dd) h1 += blk[e1];
+      if (lane < D) gv += fg[(size_t)f * 2 * D + role * D + lane];
+    }
+    const int q = diag_blk[v];
+    auto put = [&](int e, double h) {
+      if (e >= dd) return;
+      Hd64[(size_t)v * dd + e] = h;
+      if (q >= 0) Hs[(size_t)q * dd + e] = h;
+      if (e % (D + 1) == 0) {  // diagonal entries: e = D i + i
+        const double damp = diag_damping ? fmin(fmax(h, 1e-6), 1e32) : 1.0;
+        dampD[(size_t)v * D + e / (D + 1)] = damp;
+        if (q >= 0) dampS[(size_t)q * D + e / (D + 1)] = damp;
+      }
+    };
+    put(e0, h0);
+    put(e1, h1);
+    if (lane < D) g[(size_t)v * D + lane] = gv;
+    return;
+  }
+  const int64_t t = (int64_t)(blockIdx.x - var_blocks) * blockDim.x + threadIdx.x;
   if (t >= (int64_t)nblk * D) return;
   const int p = (int)(t / D), r = (int)(t % D);
   const int j = blk_col[p];
-  if (mask && !(mask[j] & 1)) return;  // (a joint batch's graph not in this round)
-  double* out = Hs + (size_t)p * dd + r * D;
-  if (blk_row[p] == j) {
-    const int v = perm[j];
+  if (blk_row[p] == j || (mask && !(mask[j] & 1))) return;  // (a joint batch's graph not in this round)
+  double acc[D];
 #pragma unroll
-    for (int c = 0; c < D; ++c) out[c] = Hd64[(size_t)v * dd + r * D + c];
-    dampS[(size_t)p * D + r] = dampD[(size_t)v * D + r];
-  } else {
-    double acc[D];
+  for (int c = 0; c < D; ++c) acc[c] = 0.0;
+  for (int u = a_ptr[p]; u < a_ptr[p + 1]; ++u) {
+    const int32_t x = a_src[u];
+    const double* H = fH64 + (size_t)(x >> 1) * 3 * dd + 2 * dd;
 #pragma unroll
-    for (int c = 0; c < D; ++c) acc[c] = 0.0;
-    for (int u = a_ptr[p]; u < a_ptr[p + 1]; ++u) {
-      const int32_t x = a_src[u];
-      const double* H = fH64 + (size_t)(x >> 1) * 3 * dd + 2 * dd;
-#pragma unroll
-      for (int c = 0; c < D; ++c) acc[c] += (x & 1) ? H[c * D + r] : H[r * D + c];
-    }
-#pragma unroll
-    for (int c = 0; c < D; ++c) out[c] = acc[c];
+    for (int c = 0; c < D; ++c) acc[c] += (x & 1) ? H[c * D + r] : H[r * D + c];
   }
+  double* out = Hs + (size_t)p * dd + r * D;
+#pragma unroll
+  for (int c = 0; c < D; ++c) out[c] = acc[c];
 }
 
 // Joint batch: the items (tasks, columns) of the graphs in the round, per
@@ -1916,6 +1945,11 @@ void CholDev::upload(CholPlan&& p, cudaStream_t st) {
   plan = std::move(p);
   levels = plan.levels();
   if (plan.tile != kTB) throw std::logic_error("chol plan tile size differs from the kernel's");
+  {
+    std::vector<int32_t> q((size_t)plan.N, -1);
+    for (int j = 0; j < plan.n_sparse; ++j) q[plan.perm[j]] = plan.col_ptr[j];
+    diag_blk.upload(q, st);
+  }
   perm.upload(plan.perm, st);
   col_ptr.upload(plan.col_ptr, st);
   blk_row.upload(plan.blk_row, st);
@@ -1970,19 +2004,18 @@ CholDev::~CholDev() {
     if (e) cudaEventDestroy(e);
 }
 
-void chol_block_hessian(SolverDev& s, CholDev& c, cudaStream_t st, const uint8_t* mask) {
-  const int nblk = (int)c.plan.blk_row.size();
-  if (nblk == 0) return;
-  const int tb = 256;
-  const int64_t n = (int64_t)nblk * c.plan.d;
-  if (s.dim == 3)
-    k_block_hessian<6><<<div_up(n, tb), tb, 0, st>>>(nblk, c.blk_row.get(), c.blk_col.get(), c.perm.get(),
-                                                    c.a_ptr.get(), c.a_src.get(), s.Hd64.get(), s.fH64.get(),
-                                                    s.dampD.get(), c.Hs.get(), c.dampS.get(), mask);
-  else
-    k_block_hessian<3><<<div_up(n, tb), tb, 0, st>>>(nblk, c.blk_row.get(), c.blk_col.get(), c.perm.get(),
-                                                    c.a_ptr.get(), c.a_src.get(), s.Hd64.get(), s.fH64.get(),
-                                                    s.dampD.get(), c.Hs.get(), c.dampS.get(), mask);
+void chol_assemble(SolverDev& s, CholDev& c, bool diagonal_damping, cudaStream_t st, const uint8_t* mask) {
+  if (s.N == 0) return;
+  const int nblk = (int)c.plan.blk_row.size(), tb = 128;
+  const int vb = div_up((int64_t)s.N * 32, tb), bb = div_up((int64_t)nblk * c.plan.d, tb);
+  auto run = [&](auto kernel) {
+    kernel<<<vb + bb, tb, 0, st>>>(s.N, vb, nblk, s.inc_ptr.get(), s.inc_fac.get(), s.inc_role.get(), s.fH64.get(),
+                                   s.fg.get(), s.Hd64.get(), s.g.get(), s.dampD.get(), diagonal_damping ? 1 : 0,
+                                   c.diag_blk.get(), c.blk_row.get(), c.blk_col.get(), c.a_ptr.get(), c.a_src.get(),
+                                   c.Hs.get(), c.dampS.get(), mask);
+  };
+  if (s.dim == 3) run(k_assemble_hessian<6>);
+  else run(k_assemble_hessian<3>);
   RPGO_LAUNCHED();
 }
 
@@ -2066,6 +2099,7 @@ void chol_enqueue(SolverDev& s, CholDev& c, double lambda, cudaStream_t st, doub
   const int grid = chol_grid(s);
   c.part.resize((size_t)2 * grid);
   CholArgs a = make_args(s, c, lambda);
+  a.out = host;
   void* args[] = {&a};
   RPGO_CUDA(cudaEventRecord(c.ev[0], st));
   if (s.dim == 3)
@@ -2074,7 +2108,6 @@ void chol_enqueue(SolverDev& s, CholDev& c, double lambda, cudaStream_t st, doub
     RPGO_CUDA(cudaLaunchCooperativeKernel((const void*)k_chol_solve<3>, grid, kThreads, args, 0, st));
   RPGO_LAUNCHED();
   RPGO_CUDA(cudaEventRecord(c.ev[1], st));
-  RPGO_CUDA(cudaMemcpyAsync(host, c.out.get(), 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
 }
 
 void chol_check_status(double status) {

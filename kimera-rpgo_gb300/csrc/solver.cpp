@@ -47,14 +47,13 @@ GpuNls::GpuNls(int dim, const std::vector<FactorRec>& graph, const FactorStore& 
 
 void GpuNls::set_weights(const std::vector<double>& w) { s_.weights.upload(w, st_); }
 
-double GpuNls::error_at_result() { return solver_error(s_, s_.x.get(), s_.weights.get(), st_); }
+double GpuNls::error_at_result() { return solver_error(s_, false, st_); }
 
 double GpuNls::error_at_result(std::vector<double>* w) {
   w->resize((size_t)s_.F);
   if (s_.F == 0) return 0.0;
   double* h = s_.pin.get(1);
-  const double* sum = enqueue_error_sum(s_, s_.x.get(), s_.weights.get(), st_);
-  RPGO_CUDA(cudaMemcpyAsync(h, sum, sizeof(double), cudaMemcpyDeviceToHost, st_));
+  enqueue_error_sum(s_, false, h, st_);
   s_.weights.download(w->data(), (size_t)s_.F, st_);
   RPGO_CUDA(cudaStreamSynchronize(st_));
   return h[0];
@@ -71,7 +70,7 @@ void GpuNls::optimize(const LmParams& p, NlsStats* st, bool from_current) {
   SolverDev& s = s_;
   if (!from_current)
     RPGO_CUDA(cudaMemcpyAsync(s.x.get(), s.x0.get(), s.x0.size() * sizeof(double), cudaMemcpyDeviceToDevice, st_));
-  double cur_err = solver_error(s, s.x.get(), s.weights.get(), st_);
+  double cur_err = solver_error(s, false, st_);
   if (cur_err <= p.error_tol || p.max_iterations <= 0) return;
   double lambda = p.lambda_initial;
   int iters = 0;
@@ -88,8 +87,8 @@ void GpuNls::optimize(const LmParams& p, NlsStats* st, bool from_current) {
         return;
       }
       solver_retract(s, st_);
-      std::swap(s.x, s.xnew);
-      cur_err = solver_error(s, s.x.get(), s.weights.get(), st_);
+      cur_err = solver_error(s, true, st_);
+      solver_accept(s);
       ++iters;
     } else {
       while (true) {
@@ -107,7 +106,7 @@ void GpuNls::optimize(const LmParams& p, NlsStats* st, bool from_current) {
           if (std::fabs(cost_change) < p.rel_tol * cur_err) stop_search = true;
         }
         if (success) {
-          std::swap(s.x, s.xnew);
+          solver_accept(s);
           cur_err = nerr;
           lambda = std::max(p.lambda_lower, lambda / p.lambda_factor);
           ++iters;

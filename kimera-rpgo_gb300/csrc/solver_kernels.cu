@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(kErrThreads) k_factor_err_sum(int F, const int
                                                         const int32_t* __restrict__ vi,
                                                         const int32_t* __restrict__ vj, const double* __restrict__ z,
                                                         const double* __restrict__ R, const double* __restrict__ x,
-                                                        const double* __restrict__ w, double* __restrict__ part,
+                                                        const double* __restrict__ w, double* __restrict__ res,
+                                                        double* __restrict__ part,
                                                         unsigned int* __restrict__ ticket, double* __restrict__ sum) {
   using L = SLie<DIM>;
   constexpr int d = L::d, st = L::stride;
@@ -119,10 +120,16 @@ __global__ void __launch_bounds__(kErrThreads) k_factor_err_sum(int F, const int
       L::load(x + (size_t)vj[f] * st, Xj);
       L::between(Xi, Xj, h);
       L::between(Z, h, rel);
+      double hv[st];
+      L::store(h, hv);
+#pragma unroll
+      for (int i = 0; i < st; ++i) res[(size_t)(d + i) * F + f] = hv[i];
     } else {
       L::between(Xi, Z, rel);
     }
     L::logmap(rel, e);
+#pragma unroll
+    for (int i = 0; i < d; ++i) res[(size_t)i * F + f] = e[i];
     const double* Rf = R + (size_t)f * d * d;
     double s2 = 0.0;
 #pragma unroll
@@ -210,16 +217,20 @@ __global__ void __launch_bounds__(128) k_linearize_a(int F, const int32_t* __res
                                                      const int32_t* __restrict__ vi, const int32_t* __restrict__ vj,
                                                      const double* __restrict__ z, const double* __restrict__ R,
                                                      const double* __restrict__ x, const double* __restrict__ w,
-                                                     double* __restrict__ rec, const uint8_t* __restrict__ mask) {
+                                                     const double* __restrict__ res, double* __restrict__ rec,
+                                                     const uint8_t* __restrict__ mask) {
   using L = SLie<DIM>;
   constexpr int d = L::d, st = L::stride, dd = d * d, RS = d + 2 * dd + 1;
   // Two warps per 32 factors (the FP64 chain of one thread is the cost, and
   // one thread per factor fills only about a quarter of the SM
   // sub-partitions; roles split by warp, not by lane, so that neither
-  // role's instructions run with half the lanes idle): the role-0 warp forms
-  // the residual, hands its log map to the role-1 warp through shared memory,
+  // role's instructions run with half the lanes idle): the role-0 warp takes
+  // the residual's log map, hands it to the role-1 warp through shared memory,
   // then forms the adjoint and the whitened residual; the role-1 warp forms
-  // the log-map Jacobian.
+  // the log-map Jacobian. With res the log map and the relative pose are those
+  // that the error sum at the same values has left there (the same operations,
+  // so the same bits); without (joint batches), role 0 evaluates them: 22 -> 14
+  // us a pass at 300 poses.
   __shared__ double sh_e[2][32][d];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = warp >> 1, role = warp & 1;
@@ -233,18 +244,29 @@ __global__ void __launch_bounds__(128) k_linearize_a(int F, const int32_t* __res
 #pragma unroll
     for (int i = 0; i < d; ++i) e[i] = 0.0;
     if (valid) {
-      typename L::Pose Xi, Z, rel;
-      L::load(x + (size_t)vi[f] * st, Xi);
-      L::load(z + (size_t)f * st, Z);
-      if (between) {
-        typename L::Pose Xj;
-        L::load(x + (size_t)vj[f] * st, Xj);
-        L::between(Xi, Xj, h);
-        L::between(Z, h, rel);
+      if (res) {
+#pragma unroll
+        for (int i = 0; i < d; ++i) e[i] = res[(size_t)i * F + f];
+        if (between) {
+          double hv[st];
+#pragma unroll
+          for (int i = 0; i < st; ++i) hv[i] = res[(size_t)(d + i) * F + f];
+          L::load(hv, h);
+        }
       } else {
-        L::between(Xi, Z, rel);
+        typename L::Pose Xi, Z, rel;
+        L::load(x + (size_t)vi[f] * st, Xi);
+        L::load(z + (size_t)f * st, Z);
+        if (between) {
+          typename L::Pose Xj;
+          L::load(x + (size_t)vj[f] * st, Xj);
+          L::between(Xi, Xj, h);
+          L::between(Z, h, rel);
+        } else {
+          L::between(Xi, Z, rel);
+        }
+        L::logmap(rel, e);
       }
-      L::logmap(rel, e);
     }
 #pragma unroll
     for (int i = 0; i < d; ++i) sh_e[pair][lane][i] = e[i];
@@ -447,38 +469,6 @@ __global__ void k_assemble(int N, const int32_t* __restrict__ inc_ptr, const int
     g[(size_t)v * D + i] = gv[i];
     dampD[(size_t)v * D + i] = diag_damping ? fmin(fmax(H[D * i + i], 1e-6), 1e32) : 1.0;
   }
-}
-
-// Assembly for the direct solver: one warp per variable, lane e owning the
-// block entries e and e + 32 (and gradient entry e < D); the same sums in the
-// same factor order as k_assemble (identical FP64 results), without the FP32
-// preconditioner blocks, which only the PCG path reads.
-template <int D>
-__global__ void k_assemble_direct(int N, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc_fac,
-                                  const int8_t* __restrict__ inc_role, const double* __restrict__ fH64,
-                                  const double* __restrict__ fg, double* __restrict__ Hd64, double* __restrict__ g,
-                                  double* __restrict__ dampD, int diag_damping, const uint8_t* __restrict__ mask) {
-  constexpr int dd = D * D;
-  const int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (v >= N || (mask && !(mask[v] & 1))) return;
-  const int e0 = lane, e1 = lane + 32;
-  double h0 = 0.0, h1 = 0.0, gv = 0.0;
-  for (int k = inc_ptr[v]; k < inc_ptr[v + 1]; ++k) {
-    const int f = inc_fac[k];
-    const int role = inc_role[k];
-    const double* blk = fH64 + (size_t)f * 3 * dd + (role == 1 ? dd : 0);
-    if (e0 < dd) h0 += blk[e0];
-    if (e1 < dd) h1 += blk[e1];
-    if (lane < D) gv += fg[(size_t)f * 2 * D + role * D + lane];
-  }
-  if (e0 < dd) Hd64[(size_t)v * dd + e0] = h0;
-  if (e1 < dd) Hd64[(size_t)v * dd + e1] = h1;
-  if (lane < D) g[(size_t)v * D + lane] = gv;
-  // diagonal entries: e = D i + i
-  if (e0 < dd && e0 % (D + 1) == 0)
-    dampD[(size_t)v * D + e0 / (D + 1)] = diag_damping ? fmin(fmax(h0, 1e-6), 1e32) : 1.0;
-  if (e1 < dd && e1 % (D + 1) == 0)
-    dampD[(size_t)v * D + e1 / (D + 1)] = diag_damping ? fmin(fmax(h1, 1e-6), 1e32) : 1.0;
 }
 
 // ------------------------------------------------------------------ small dense (FP32)
@@ -768,6 +758,8 @@ void solver_upload(SolverDev& s, int dim, const std::vector<int32_t>& kind, cons
   s.fH64.resize((size_t)F * 3 * dd);
   s.fg.resize((size_t)F * 2 * d);
   s.ferr.resize(F);
+  s.res.resize((size_t)F * (d + s.stride));
+  s.resnew.resize((size_t)F * (d + s.stride));
   s.Hd.resize((size_t)N * dd);
   s.Hd64.resize((size_t)N * dd);
   s.Md.resize((size_t)N * dd);
@@ -821,33 +813,35 @@ void solver_upload(SolverDev& s, int dim, const std::vector<int32_t>& kind, cons
   }
 }
 
-// enqueue k_factor_err_sum: the sum lands in s.red[blocks]
-double* enqueue_error_sum(SolverDev& s, const double* x, const double* weights, cudaStream_t st) {
+void enqueue_error_sum(SolverDev& s, bool at_new, double* host, cudaStream_t st) {
   const int blocks = std::min(1024, div_up(s.F, kErrThreads));
   if (s.ticket.size() == 0) {
     s.ticket.resize(1);
     s.ticket.zero(st);
   }
-  s.red.resize(blocks + 1);
-  if (s.dim == 3)
-    k_factor_err_sum<3><<<blocks, kErrThreads, 0, st>>>(s.F, s.kind.get(), s.vi.get(), s.vj.get(), s.z.get(),
-                                                s.sqrt_info.get(), x, weights, s.red.get(), s.ticket.get(),
-                                                s.red.get() + blocks);
-  else
-    k_factor_err_sum<2><<<blocks, kErrThreads, 0, st>>>(s.F, s.kind.get(), s.vi.get(), s.vj.get(), s.z.get(),
-                                                s.sqrt_info.get(), x, weights, s.red.get(), s.ticket.get(),
-                                                s.red.get() + blocks);
+  s.red.resize(blocks);
+  const double* x = at_new ? s.xnew.get() : s.x.get();
+  double* res = at_new ? s.resnew.get() : s.res.get();
+  auto run = [&](auto kernel) {
+    kernel<<<blocks, kErrThreads, 0, st>>>(s.F, s.kind.get(), s.vi.get(), s.vj.get(), s.z.get(), s.sqrt_info.get(), x,
+                                           s.weights.get(), res, s.red.get(), s.ticket.get(), host);
+  };
+  if (s.dim == 3) run(k_factor_err_sum<3>);
+  else run(k_factor_err_sum<2>);
   RPGO_LAUNCHED();
-  return s.red.get() + blocks;
 }
 
-double solver_error(SolverDev& s, const double* x, const double* weights, cudaStream_t st) {
+double solver_error(SolverDev& s, bool at_new, cudaStream_t st) {
   if (s.F == 0) return 0.0;
-  const double* sum = enqueue_error_sum(s, x, weights, st);
-  double h = 0.0;
-  RPGO_CUDA(cudaMemcpyAsync(&h, sum, sizeof(double), cudaMemcpyDeviceToHost, st));
+  double* h = s.pin.get(3);
+  enqueue_error_sum(s, at_new, h + 2, st);
   RPGO_CUDA(cudaStreamSynchronize(st));
-  return h;
+  return h[2];
+}
+
+void solver_accept(SolverDev& s) {
+  std::swap(s.x, s.xnew);
+  std::swap(s.res, s.resnew);
 }
 
 void solver_factor_errors(SolverDev& s, const double* x, std::vector<double>* out, cudaStream_t st) {
@@ -871,38 +865,23 @@ void solver_linearize(SolverDev& s, bool diagonal_damping, cudaStream_t st) {
     const int d = s.d, rs = d + 2 * d * d + 1;
     s.lin_rec.resize((size_t)s.F * rs);
     const int per_block = 4 * (32 / d);  // k_linearize_b: 4 warps of 32/d factors
-    if (s.dim == 3) {
-      k_linearize_a<3><<<div_up(s.F, 64), 128, 0, st>>>(s.F, s.kind.get(), s.vi.get(), s.vj.get(), s.z.get(),
-                                                       s.sqrt_info.get(), s.x.get(), s.weights.get(), s.lin_rec.get(), nullptr);
+    auto run = [&](auto a, auto b) {
+      a<<<div_up(s.F, 64), 128, 0, st>>>(s.F, s.kind.get(), s.vi.get(), s.vj.get(), s.z.get(), s.sqrt_info.get(),
+                                         s.x.get(), s.weights.get(), s.res.get(), s.lin_rec.get(), nullptr);
       RPGO_LAUNCHED();
-      k_linearize_b<3><<<div_up(s.F, per_block), 128, 0, st>>>(s.F, s.kind.get(), s.sqrt_info.get(), s.lin_rec.get(),
-                                                               need_pcg(s) ? s.fH.get() : nullptr, s.fH64.get(),
-                                                               s.fg.get(), nullptr);
-    } else {
-      k_linearize_a<2><<<div_up(s.F, 64), 128, 0, st>>>(s.F, s.kind.get(), s.vi.get(), s.vj.get(), s.z.get(),
-                                                       s.sqrt_info.get(), s.x.get(), s.weights.get(), s.lin_rec.get(), nullptr);
+      b<<<div_up(s.F, per_block), 128, 0, st>>>(s.F, s.kind.get(), s.sqrt_info.get(), s.lin_rec.get(),
+                                                need_pcg(s) ? s.fH.get() : nullptr, s.fH64.get(), s.fg.get(),
+                                                nullptr);
       RPGO_LAUNCHED();
-      k_linearize_b<2><<<div_up(s.F, per_block), 128, 0, st>>>(s.F, s.kind.get(), s.sqrt_info.get(), s.lin_rec.get(),
-                                                               need_pcg(s) ? s.fH.get() : nullptr, s.fH64.get(),
-                                                               s.fg.get(), nullptr);
-    }
-    RPGO_LAUNCHED();
+    };
+    if (s.dim == 3) run(k_linearize_a<3>, k_linearize_b<3>);
+    else run(k_linearize_a<2>, k_linearize_b<2>);
   }
   if (use_direct(s)) {
-    const int blocks = div_up((int64_t)s.N * 32, tb);
-    if (s.dim == 3)
-      k_assemble_direct<6><<<blocks, tb, 0, st>>>(s.N, s.inc_ptr.get(), s.inc_fac.get(), s.inc_role.get(),
-                                                  s.fH64.get(), s.fg.get(), s.Hd64.get(), s.g.get(), s.dampD.get(),
-                                                  diagonal_damping ? 1 : 0, nullptr);
-    else
-      k_assemble_direct<3><<<blocks, tb, 0, st>>>(s.N, s.inc_ptr.get(), s.inc_fac.get(), s.inc_role.get(),
-                                                  s.fH64.get(), s.fg.get(), s.Hd64.get(), s.g.get(), s.dampD.get(),
-                                                  diagonal_damping ? 1 : 0, nullptr);
-    RPGO_LAUNCHED();
-    chol_block_hessian(s, *s.chol, st);
+    chol_assemble(s, *s.chol, diagonal_damping, st);
     if (!s.race) return;
     // racing: the PCG path's blocks too (same FP64 diagonal, gradient and
-    // damping as k_assemble_direct's)
+    // damping as chol_assemble's)
   }
   if (s.dim == 3)
     k_assemble<6><<<div_up(s.N, tb), tb, 0, st>>>(s.N, s.inc_ptr.get(), s.inc_fac.get(), s.inc_role.get(),
@@ -1380,7 +1359,7 @@ SolveOut solver_solve_eval(SolverDev& s, double lambda, cudaStream_t st, double*
     SolveOut o = solver_solve(s, lambda, st);
     if (o.ok && o.lin_change >= 0.0) {
       solver_retract(s, st);
-      *nerr = solver_error(s, s.xnew.get(), s.weights.get(), st);
+      *nerr = solver_error(s, true, st);
     }
     return o;
   }
@@ -1390,10 +1369,7 @@ SolveOut solver_solve_eval(SolverDev& s, double lambda, cudaStream_t st, double*
   // when it failed)
   solver_retract(s, st);
   host[2] = 0.0;
-  if (s.F > 0) {
-    const double* sum = enqueue_error_sum(s, s.xnew.get(), s.weights.get(), st);
-    RPGO_CUDA(cudaMemcpyAsync(host + 2, sum, sizeof(double), cudaMemcpyDeviceToHost, st));
-  }
+  if (s.F > 0) enqueue_error_sum(s, true, host + 2, st);
   RPGO_CUDA(cudaStreamSynchronize(st));
   SolveOut o = chol_finish(s, *s.chol, host);
   *nerr = host[2];
@@ -1456,16 +1432,12 @@ static void batch_pre_t(SolverDev& s, BatchDev& b, bool diagonal_damping, bool a
   s.lin_rec.resize((size_t)F * rs);
   k_linearize_a<DIM><<<div_up(F, 64), 128, 0, st>>>(F, s.kind.get(), s.vi.get(), s.vj.get(), s.z.get(),
                                                                 s.sqrt_info.get(), s.x.get(), s.weights.get(),
-                                                                s.lin_rec.get(), b.fmask.get());
+                                                                nullptr, s.lin_rec.get(), b.fmask.get());
   RPGO_LAUNCHED();
   k_linearize_b<DIM><<<div_up(F, 4 * (32 / d)), 128, 0, st>>>(F, s.kind.get(), s.sqrt_info.get(), s.lin_rec.get(),
                                                               nullptr, s.fH64.get(), s.fg.get(), b.fmask.get());
   RPGO_LAUNCHED();
-  k_assemble_direct<d><<<div_up((int64_t)N * 32, tb), tb, 0, st>>>(
-      N, s.inc_ptr.get(), s.inc_fac.get(), s.inc_role.get(), s.fH64.get(), s.fg.get(), s.Hd64.get(), s.g.get(),
-      s.dampD.get(), diagonal_damping ? 1 : 0, b.vmask.get());
-  RPGO_LAUNCHED();
-  chol_block_hessian(s, *s.chol, st, b.vmask.get());
+  chol_assemble(s, *s.chol, diagonal_damping, st, b.vmask.get());
 }
 
 template <int DIM>

@@ -79,6 +79,9 @@ struct SolverDev {
   DeviceBuffer<double> x0, x, xnew;  // N x stride
   DeviceBuffer<double> delta;        // N x d
   DeviceBuffer<double> ferr;         // F (per-factor error)
+  // per factor the residual's log map and the relative pose X_i^-1 X_j, as the
+  // error sum at x (at xnew) evaluated them: [value][factor], d + stride values
+  DeviceBuffer<double> res, resnew;
   DeviceBuffer<double> red;          // reduction scratch
   DeviceBuffer<unsigned int> ticket; // last-block counter of the one-launch error sum
   // preconditioner (block cyclic reduction) and CG scratch
@@ -111,11 +114,13 @@ struct SolveOut {
 void solver_upload(SolverDev& s, int dim, const std::vector<int32_t>& kind, const std::vector<int32_t>& vi,
                    const std::vector<int32_t>& vj, int N, cudaStream_t st, bool direct,
                    CholPlan* plan = nullptr);
-// per-factor error 0.5 w |R e|^2 at values `x` (weights null = 1); returns the sum
-double solver_error(SolverDev& s, const double* x, const double* weights, cudaStream_t st);
+// sum of the factors' errors 0.5 w |R e|^2 at s.x (at_new: at s.xnew) with
+// s.weights; leaves the residuals there in s.res (s.resnew)
+double solver_error(SolverDev& s, bool at_new, cudaStream_t st);
 // per-factor unweighted errors at x into s.ferr (host copy returned)
 void solver_factor_errors(SolverDev& s, const double* x, std::vector<double>* out, cudaStream_t st);
-// linearise at s.x with s.weights; assembles Hd, g, tree blocks, damping diagonal
+// linearise at s.x with s.weights; the last solver_error evaluated s.x (or the
+// accepted s.xnew); assembles Hd, g, tree blocks, damping diagonal
 void solver_linearize(SolverDev& s, bool diagonal_damping, cudaStream_t st);
 // solve (H + lambda D) delta = -g into s.delta
 SolveOut solver_solve(SolverDev& s, double lambda, cudaStream_t st);
@@ -130,9 +135,11 @@ double set_direct_solve_guard(double flops, int prefer);
 SolveOut solver_solve_eval(SolverDev& s, double lambda, cudaStream_t st, double* nerr);
 // xnew = x (+) delta
 void solver_retract(SolverDev& s, cudaStream_t st);
-// enqueue the weighted error of x (one launch); returns the device word that
-// will hold it
-double* enqueue_error_sum(SolverDev& s, const double* x, const double* weights, cudaStream_t st);
+// enqueue solver_error (one launch); the kernel writes the sum to *host
+// (page-locked)
+void enqueue_error_sum(SolverDev& s, bool at_new, double* host, cudaStream_t st);
+// the candidate becomes the estimate (values and residuals)
+void solver_accept(SolverDev& s);
 // TLS weights (GncOptimizer::calculateWeights) for factors >= n_known, with
 // the per-factor thresholds barc on the device; enqueued only (the stream
 // orders them before the next solve)
