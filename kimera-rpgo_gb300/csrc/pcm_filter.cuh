@@ -1,4 +1,4 @@
-// Decides most pairwise consistency tests of 3D uncertain poses
+// Decides most pairwise consistency tests of uncertain poses (3D, 2D)
 // (Pcm::areLoopsConsistent, include/KimeraRPGO/outlier/Pcm.h:670-718) in FP32
 // arithmetic, with a bound on its own error; the rest is left to the exact
 // FP64 test of pcm_kernels.cu. Host and device code: the tests run it on the
@@ -584,6 +584,35 @@ RPGO_HD bool logmap(const Pose& T, float (&xi)[6], float& ew, float& et) {
   return ok;
 }
 
+// The verdict from the computed d^2, y.x and y^T C y, the sums p.|y|, e.|y|,
+// p.sqrt(C^-1_ii), e.sqrt(C^-1_ii) and the error eta of the two `between`.
+RPGO_HD int decide(float d2, float yx, float yCy, float py, float ey, float ph, float eh, float eta, float th2) {
+  // the covariances of the two `between` (eta), 16 roundings in each of three
+  // compositions, 10 in the factorisation and in y^T C y; what was computed
+  // from them with a margin of 1.1
+  const float eps = fmulf(1.1f, fadd(eta, 64.f * kU));
+  const float low = fsub(fsub(fmulf(2.f, yx), yCy), ffma(eps, fmulf(py, py), fmulf(2.2f, ey)));
+  if (low > fmulf(th2, 1.f + 16.f * kU)) return 0;
+  const float kap = fmulf(eps, fmulf(ph, ph));
+  const float d = fadd(fmulf(fsqr(d2), 1.f + 64.f * kU), fmulf(1.1f, eh));
+  const float top = fmulf(th2, 1.f - 16.f * kU);
+  if (kap < 0.9f && fmulf(d, d) < fmulf(top, fsub(1.f, kap))) return 1;
+  // nearer to the threshold: the lower bound's terms, to first order in kap
+  const float up = ffma(1.5f, ffma(eps, fmulf(py, py), ffma(2.f, ey, fmulf(eh, eh))), fmulf(d2, 1.f + 64.f * kU));
+  return kap < 0.125f && up < top ? 1 : 2;
+}
+
+// The translations that the pose chain goes through (1-norms); the loop's
+// translation has at most kPoseErr of their sum as error from the chain (about
+// 40 roundings of 2^-48, and a margin of 6).
+constexpr float kPoseErr = 9.094947017729282e-13f;  // 2^-40
+template <int D>
+RPGO_HD float chain_length(const Item& I, const Item& J, int ta, int tb, int zt) {
+  float s = fadd(fadd(I.g(ta), I.g(tb)), fadd(J.g(ta), J.g(tb)));
+  for (int a = 0; a < D; ++a) s = fadd(s, fadd(fabsv(I.g(zt + a)), fabsv(J.g(zt + a))));
+  return s;
+}
+
 // The verdict on closures i and j (flip: the group stores them in opposite
 // directions, so j's endpoints change places) against the threshold's square:
 // 0 inconsistent, 1 consistent, 2 unsure. No early returns: every thread of a
@@ -648,6 +677,7 @@ RPGO_HD int verdict(const Group& g, int i, int j, bool flip, float th2, Sync syn
   compose(Q, P, L);
   float xi[6], ew, et;
   ok &= logmap(L, xi, ew, et);
+  et = ffma(kPoseErr, chain_length<3>(I, J, kTA, kTB1, kZt), et);
   // d^2 = x^T C^-1 x: L z = x, y = L^-T D^-1 z
   float F[15], W[15], iD[6], h[6];
   ok &= factor(S, F, W, iD, h);
@@ -683,20 +713,313 @@ RPGO_HD int verdict(const Group& g, int i, int j, bool flip, float th2, Sync syn
     yCy = ffma(2.f * c, y[a], yCy);
   }
   if (!ok) return 2;
-  // the covariances of the two `between` (eta), 16 roundings in each of three
-  // compositions, 10 in the factorisation and in y^T C y; what was computed
-  // from them with a margin of 1.1
-  const float eps = fmulf(1.1f, fadd(eta, 64.f * kU));
-  const float low = fsub(fsub(fmulf(2.f, yx), yCy), ffma(eps, fmulf(py, py), fmulf(2.2f, ey)));
-  if (low > fmulf(th2, 1.f + 16.f * kU)) return 0;
-  const float kap = fmulf(eps, fmulf(ph, ph));
-  const float d = fadd(fmulf(fsqr(d2), 1.f + 64.f * kU), fmulf(1.1f, eh));
-  const float top = fmulf(th2, 1.f - 16.f * kU);
-  if (kap < 0.9f && fmulf(d, d) < fmulf(top, fsub(1.f, kap))) return 1;
-  // nearer to the threshold: the lower bound's terms, to first order in kap
-  const float up = ffma(1.5f, ffma(eps, fmulf(py, py), ffma(2.f, ey, fmulf(eh, eh))), fmulf(d2, 1.f + 64.f * kU));
-  return kap < 0.125f && up < top ? 1 : 2;
+  return decide(d2, yx, yCy, py, ey, ph, eh, eta, th2);
 }
+
+// ------------------------------------------------------------------ 2D
+// The same test for Pose2: tangent (v_x, v_y, omega), Ad = [[R, (y, -x)], [0, 1]].
+// Bounds as in 3D, with fewer terms; a covariance as its lower triangle
+// (xx, yx, yy, wx, wy, ww).
+constexpr int kPairs2 = 24;   // pose a (c, s, x, y), cov a, pose b, cov b, measured pose
+constexpr int kFloats2 = 19;  // inverse measurement's (x, y), its covariance (6), sqrt of its diagonal (3), sqrt of
+                              // the diagonals of cov a and cov b (3 each), |t_a|, |t_b|
+constexpr int kCov2 = 4, kPoseB2 = 10, kPoseZ2 = 20;
+constexpr int kZt2 = 0, kZc2 = 2, kZg2 = 8, kGA2 = 11, kGB2 = 14, kTA2 = 17, kTB2 = 18;
+
+RPGO_HD int tri_full2(int e) {
+  int i = 0;
+  while (e > i) e -= ++i;
+  return 3 * i + e;
+}
+RPGO_HD D2 pack_pair2(int v, const double* pa, const double* ca, const double* pb, const double* cb,
+                      const double* zp) {
+  if (v < kCov2) return split(pa[v]);
+  if (v < kPoseB2) return split(ca[tri_full2(v - kCov2)]);
+  if (v < kPoseB2 + kCov2) return split(pb[v - kPoseB2]);
+  if (v < kPoseZ2) return split(cb[tri_full2(v - kPoseB2 - kCov2)]);
+  return split(zp[v - kPoseZ2]);
+}
+RPGO_HD float pack_float2(int v, const double* pa, const double* ca, const double* pb, const double* cb,
+                          const double* zp, const double* zc) {
+  if (v == 0) return (float)-(zp[0] * zp[2] + zp[1] * zp[3]);
+  if (v == 1) return (float)-(zp[0] * zp[3] - zp[1] * zp[2]);
+  if (v < kZg2) return (float)zc[tri_full2(v - kZc2)];
+  if (v < kGA2) return fsqr((float)zc[4 * (v - kZg2)]);
+  if (v < kGB2) return fsqr((float)ca[4 * (v - kGA2)]);
+  if (v < kTA2) return fsqr((float)cb[4 * (v - kGB2)]);
+  const double* t = (v == kTA2 ? pa : pb) + 2;
+  return (float)(std::fabs(t[0]) + std::fabs(t[1]));
+}
+RPGO_HD bool cov_premise2(const double* c, bool whole) {
+  bool ok = true;
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j <= i; ++j) {
+      const double x = c[3 * i + j], b = c[4 * i] * c[4 * j];
+      ok = ok && x * x <= 1.0001 * b && (!whole || c[3 * j + i] == x) && c[4 * i] >= 0.0 && c[4 * i] < 1e15;
+    }
+  return ok;
+}
+RPGO_HD bool pose_premise2(const double* p) {
+  return std::fabs(p[0] * p[0] + p[1] * p[1] - 1.0) < 1e-7 && std::fabs(p[2]) < 1e12 && std::fabs(p[3]) < 1e12;
+}
+
+RPGO_HD D2 dot2(D2 a0, D2 a1, D2 b0, D2 b1) {
+  Acc x = acc_mul(a0, b0);
+  acc_fma(x, a1, b1);
+  return norm(x);
+}
+RPGO_HD D2 fma2(D2 a, D2 b, D2 v) {
+  Acc x{v.h, v.l};
+  acc_fma(x, a, b);
+  return norm(x);
+}
+RPGO_HD float dot2(float a0, float a1, float b0, float b1) { return ffma(a1, b1, fmulf(a0, b0)); }
+RPGO_HD float fma2(float a, float b, float v) { return ffma(a, b, v); }
+RPGO_HD float neg(float a) { return -a; }
+
+// Ad S Ad^T for rotation (c, s) and r = (y, -x) (lower triangles)
+template <class T>
+RPGO_HD void congruence2(T c, T s, T r0, T r1, const T* S, T* C) {
+  const T m00 = dot2(c, neg(s), S[0], S[1]), m01 = dot2(c, neg(s), S[1], S[2]);
+  const T m10 = dot2(s, c, S[0], S[1]), m11 = dot2(s, c, S[1], S[2]);
+  const T b0 = dot2(c, neg(s), S[3], S[4]), b1 = dot2(s, c, S[3], S[4]);
+  C[5] = S[5];
+  C[3] = fma2(r0, S[5], b0);
+  C[4] = fma2(r1, S[5], b1);
+  C[0] = fma2(b0, r0, fma2(r0, C[3], dot2(m00, m01, c, neg(s))));
+  C[1] = fma2(b1, r0, fma2(r1, C[3], dot2(m10, m11, c, neg(s))));
+  C[2] = fma2(b1, r1, fma2(r1, C[4], dot2(m10, m11, s, c)));
+}
+
+struct Pose2D {
+  D2 c, s, x, y;
+};
+RPGO_HD Pose2D load_pose2(const Item& i, int v) { return Pose2D{i.d(v), i.d(v + 1), i.d(v + 2), i.d(v + 3)}; }
+RPGO_HD Pose2D compose2(const Pose2D& A, const Pose2D& B) {
+  Acc x{A.x.h, A.x.l}, y{A.y.h, A.y.l};
+  acc_fma(x, A.c, B.x);
+  acc_fma(x, neg(A.s), B.y);
+  acc_fma(y, A.s, B.x);
+  acc_fma(y, A.c, B.y);
+  return Pose2D{dot2(A.c, neg(A.s), B.c, B.s), dot2(A.s, A.c, B.c, B.s), norm(x), norm(y)};
+}
+RPGO_HD Pose2D inverse2(const Pose2D& A) {
+  return Pose2D{A.c, neg(A.s), neg(dot2(A.c, A.s, A.x, A.y)), neg(dot2(A.c, neg(A.s), A.y, A.x))};
+}
+RPGO_HD Pose2D between2(const Pose2D& A, const Pose2D& B) {
+  const D2 dx = sub(B.x, A.x), dy = sub(B.y, A.y);
+  return Pose2D{dot2(A.c, A.s, B.c, B.s), dot2(A.c, neg(A.s), B.s, B.c), dot2(A.c, A.s, dx, dy),
+                dot2(A.c, neg(A.s), dy, dx)};
+}
+
+// LDL^T (see factor): L and L^-1 as (10, 20, 21)
+RPGO_HD bool factor2(const float* S, float (&L)[3], float (&W)[3], float (&iD)[3], float (&h)[3]) {
+  iD[0] = fdvd(1.f, S[0]);
+  L[0] = fmulf(S[1], iD[0]);
+  const float d1 = ffma(-S[1], L[0], S[2]);
+  iD[1] = fdvd(1.f, d1);
+  L[1] = fmulf(S[3], iD[0]);
+  const float e = ffma(-S[3], L[0], S[4]);
+  L[2] = fmulf(e, iD[1]);
+  const float d2 = ffma(-e, L[2], ffma(-S[3], L[1], S[5]));
+  iD[2] = fdvd(1.f, d2);
+  W[0] = -L[0];
+  W[2] = -L[2];
+  W[1] = ffma(-L[2], W[0], -L[1]);
+  h[0] = ffma(fmulf(W[1], W[1]), iD[2], ffma(fmulf(W[0], W[0]), iD[1], iD[0]));
+  h[1] = ffma(fmulf(W[2], W[2]), iD[2], iD[1]);
+  h[2] = iD[2];
+  return S[0] > 0.f && d1 > 0.f && d2 > 0.f;
+}
+
+RPGO_HD bool between_cov2(const Item& x, int va, int ga, int ta, const Item& y, int vc, int gc, int tc, Pose2D& pose,
+                          float (&S)[6], float (&s)[3], float& eta) {
+  const Pose2D A = load_pose2(x, va), B = load_pose2(y, vc);
+  pose = between2(A, B);
+  const float gv = fadd(x.g(ga), x.g(ga + 1)), hv = fadd(y.g(gc), y.g(gc + 1));
+  const float qw = fadd(x.g(ga + 2), y.g(gc + 2));
+  const float lever =
+      fadd(fadd(fabsv(pose.x.h), fabsv(pose.y.h)), fadd(fadd(x.g(ta), y.g(tc)), fadd(x.g(ta), y.g(tc))));
+  const float qv = ffma(lever, qw, fadd(gv, hv));
+  // Ad of the inverse: rotation (c, -s), r = (y', -x') of the inverse's
+  // translation; first for the main formula's first pivot, cov(v_x, v_x)
+  const Pose2D im = inverse2(pose);
+  bool main, known;
+  {
+    D2 Sx[6];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) Sx[e] = x.d(va + kCov2 + e);
+    const D2 c = im.c, ns = neg(im.s), r0 = im.y;
+    const D2 m0 = dot2(c, ns, Sx[0], Sx[1]), m1 = dot2(c, ns, Sx[1], Sx[2]), b0 = dot2(c, ns, Sx[3], Sx[4]);
+    const D2 c3 = fma2(r0, Sx[5], b0);
+    const D2 piv = sub(y.d(vc + kCov2), fma2(b0, r0, fma2(r0, c3, dot2(m0, m1, c, ns))));
+    const float e = fmulf(kDf, fmulf(qv, qv));
+    main = piv.h > e;
+    known = main || piv.h < -e;
+  }
+  const Item& X = main ? x : y;
+  const Item& Y = main ? y : x;
+  const int vX = main ? va : vc, vY = main ? vc : va;
+  const Pose2D ib = inverse2(between2(B, A));
+  const D2 c = main ? im.c : ib.c, sn = main ? im.s : ib.s, r0 = main ? im.y : ib.y, r1 = neg(main ? im.x : ib.x);
+  D2 SX[6], C[6];
+#pragma unroll
+  for (int e = 0; e < 6; ++e) SX[e] = X.d(vX + kCov2 + e);
+  congruence2(c, sn, r0, r1, SX, C);
+#pragma unroll
+  for (int e = 0; e < 6; ++e) S[e] = lo(sub(Y.d(vY + kCov2 + e), C[e]));
+  float L[3], W[3], iD[3], h[3];
+  bool ok = factor2(S, L, W, iD, h) && known;
+  const float dg[3] = {S[0], S[2], S[5]};
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    ok = ok && dg[i] > 1e-24f;
+    s[i] = fsqr(dg[i]);
+    sum = fadd(sum, fsqr(fmulf(dg[i], h[i])));
+  }
+  const float ev = fdvd(fmulf(qv, qv), dg[0] < dg[1] ? dg[0] : dg[1]), ew = fdvd(fmulf(qw, qw), dg[2]);
+  eta = ffma(kDf, ev > ew ? ev : ew, 16.f * kU);
+  return ok && fmulf(eta, fmulf(sum, sum)) < 0.5f;
+}
+
+RPGO_HD void compose_cov2(float c, float sn, float r0, float r1, float (&S)[6], float (&p)[3], const float* Z,
+                          const float* g) {
+  float C[6];
+  congruence2(c, sn, r0, r1, S, C);
+#pragma unroll
+  for (int e = 0; e < 6; ++e) S[e] = fadd(C[e], Z[e]);
+  const float ac = fabsv(c), as = fabsv(sn), v0 = p[0], v1 = p[1];
+  p[0] = fadd(ffma(fabsv(r0), p[2], ffma(as, v1, fmulf(ac, v0))), g[0]);
+  p[1] = fadd(ffma(fabsv(r1), p[2], ffma(ac, v1, fmulf(as, v0))), g[1]);
+  p[2] = fadd(p[2], g[2]);
+}
+
+template <class Sync = NoSync>
+RPGO_HD int verdict2(const Group& g, int i, int j, bool flip, float th2, Sync sync = Sync()) {
+  bool ok = g.ok[i] && g.ok[j];
+  const Item I = item(g, i), J = item(g, j);
+  Pose2D Q, P;
+  float S[6], p[3], eta = 0.f;
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const bool jb = flip != (side == 1);  // j's second endpoint
+    float SB[6], sb[3], e;
+    sync();
+    ok &= between_cov2(I, side ? kPoseB2 : 0, side ? kGB2 : kGA2, side ? kTB2 : kTA2, J, jb ? kPoseB2 : 0,
+                       jb ? kGB2 : kGA2, jb ? kTB2 : kTA2, P, SB, sb, e);
+    eta = e > eta ? e : eta;
+    if (side == 0) {
+      // (A o Z_j)^-1 o Z_i
+#pragma unroll
+      for (int a = 0; a < 6; ++a) S[a] = SB[a];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) p[a] = sb[a];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const Item& z = k ? I : J;
+        const Pose2D Z = load_pose2(z, kPoseZ2), T = compose2(P, Z);
+        float zc[6], zg[3];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) zc[a] = z.g(kZc2 + a);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) zg[a] = z.g(kZg2 + a);
+        compose_cov2(Z.c.h, -Z.s.h, z.g(kZt2 + 1), -z.g(kZt2), S, p, zc, zg);
+        if (k) Q = T;
+        else P = inverse2(T);
+      }
+    } else {
+      const Pose2D ib = inverse2(P);  // loop = Q o B
+      compose_cov2(ib.c.h, ib.s.h, ib.y.h, -ib.x.h, S, p, SB, sb);
+    }
+  }
+  const Pose2D T = compose2(Q, P);
+  // Log map. 1 - c comes from the pair, so that it keeps its digits for small
+  // angles; its error of about 2^-43 counts by 1 / angle. Below 1e-10 the
+  // exact test takes the translation itself; up to 1e-8 the pair is unsure.
+  const float c = T.c.h, s = T.s.h, x = T.x.h, y = T.y.h;
+  const float th = atan2f(s, c), at = fabsv(th), omc = fsub(fsub(1.f, c), T.c.l);
+  const bool none = at < 0.9e-10f;
+  ok = ok && fabsv(fsub(ffma(c, c, fmulf(s, s)), 1.f)) < 1e-6f && (c > 0.f || fabsv(s) > 64.f * kU) &&
+       (none || at > 1e-8f);
+  const float k = fdvd(th, ffma(s, s, fmulf(omc, omc)));
+  const float a = none ? 1.f : fmulf(k, s), b = none ? 0.f : fmulf(k, omc);
+  const float xi[3] = {ffma(b, y, fmulf(a, x)), ffma(-b, x, fmulf(a, y)), th};
+  const float et = ffma(kPoseErr, chain_length<2>(I, J, kTA2, kTB2, kZt2),
+                        fmulf(fadd(64.f * kU, none ? 0.f : fdvd(kPoseErr, at)), fadd(fabsv(x), fabsv(y))));
+  const float ew = ffma(16.f * kU, at, 1e-10f);
+  float L[3], W[3], iD[3], h[3];
+  ok &= factor2(S, L, W, iD, h);
+  const float z0 = xi[0], z1 = ffma(-L[0], z0, xi[1]), z2 = ffma(-L[2], z1, ffma(-L[1], z0, xi[2]));
+  const float d0 = fmulf(z0, iD[0]), d1 = fmulf(z1, iD[1]), d2y = fmulf(z2, iD[2]);
+  const float d2 = ffma(d2y, z2, ffma(d1, z1, fmulf(d0, z0)));
+  const float y2 = d2y, y1 = ffma(-L[2], y2, d1), y0 = ffma(-L[1], y2, ffma(-L[0], y1, d0));
+  const float yv[3] = {y0, y1, y2}, dg[3] = {S[0], S[2], S[5]};
+  float py = 0.f, ey = 0.f, ph = 0.f, eh = 0.f, yx = 0.f;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const float e = q < 2 ? et : ew, sh = fsqr(h[q]), ay = fabsv(yv[q]);
+    py = ffma(p[q], ay, py);
+    ey = ffma(e, ay, ey);
+    ph = ffma(p[q], sh, ph);
+    eh = ffma(e, sh, eh);
+    ok = ok && dg[q] > 1e-24f && p[q] < 1e15f;
+    yx = ffma(yv[q], xi[q], yx);
+  }
+  // C y
+  const float s0 = ffma(S[3], y2, ffma(S[1], y1, fmulf(S[0], y0)));
+  const float s1 = ffma(S[4], y2, ffma(S[2], y1, fmulf(S[1], y0)));
+  const float s2 = ffma(S[5], y2, ffma(S[4], y1, fmulf(S[3], y0)));
+  const float yCy = ffma(y2, s2, ffma(y1, s1, fmulf(y0, s0)));
+  if (!ok) return 2;
+  return decide(d2, yx, yCy, py, ey, ph, eh, eta, th2);
+}
+
+// ------------------------------------------------------------------ both
+template <int DIM>
+struct Filter;
+template <>
+struct Filter<3> {
+  static constexpr int pairs = kPairs, floats = kFloats;
+  RPGO_HD static D2 pair(int v, const double* pa, const double* ca, const double* pb, const double* cb,
+                         const double* z) {
+    return pack_pair(v, pa, ca, pb, cb, z);
+  }
+  RPGO_HD static float single(int v, const double* pa, const double* ca, const double* pb, const double* cb,
+                              const double* z, const double* c) {
+    return pack_float(v, pa, ca, pb, cb, z, c);
+  }
+  RPGO_HD static bool premise(const double* pa, const double* ca, const double* pb, const double* cb,
+                              const double* z, const double* c) {
+    return cov_premise(ca, true) && cov_premise(cb, true) && cov_premise(c, false) && pose_premise(pa) &&
+           pose_premise(pb) && pose_premise(z);
+  }
+  template <class Sync = NoSync>
+  RPGO_HD static int test(const Group& g, int i, int j, bool flip, float th2, Sync sync = Sync()) {
+    return verdict(g, i, j, flip, th2, sync);
+  }
+};
+template <>
+struct Filter<2> {
+  static constexpr int pairs = kPairs2, floats = kFloats2;
+  RPGO_HD static D2 pair(int v, const double* pa, const double* ca, const double* pb, const double* cb,
+                         const double* z) {
+    return pack_pair2(v, pa, ca, pb, cb, z);
+  }
+  RPGO_HD static float single(int v, const double* pa, const double* ca, const double* pb, const double* cb,
+                              const double* z, const double* c) {
+    return pack_float2(v, pa, ca, pb, cb, z, c);
+  }
+  RPGO_HD static bool premise(const double* pa, const double* ca, const double* pb, const double* cb,
+                              const double* z, const double* c) {
+    return cov_premise2(ca, true) && cov_premise2(cb, true) && cov_premise2(c, false) && pose_premise2(pa) &&
+           pose_premise2(pb) && pose_premise2(z);
+  }
+  template <class Sync = NoSync>
+  RPGO_HD static int test(const Group& g, int i, int j, bool flip, float th2, Sync sync = Sync()) {
+    return verdict2(g, i, j, flip, th2, sync);
+  }
+};
 
 }  // namespace pf
 }  // namespace rpgo

@@ -632,51 +632,53 @@ __global__ void __launch_bounds__(32 * ROWS) k_pairwise(int n, int row_begin, co
   if (lane == 0) lower[(size_t)(j - row_begin) * words + blockIdx.x] = bits;
 }
 
-// The 3D PoseWithCovariance test of many pairs: FP32 with an error bound
+// The PoseWithCovariance test of many pairs: FP32 with an error bound
 // decides about 99 % of them (pcm_filter.cuh), the exact FP64 test the rest.
 // The FP64 pipe issues a warp instruction in 64 cycles, FP32 in one, and a
 // `between` in pairs of FP32 costs about 12 FP32 instructions per FP64 FMA:
 // 10,400 instructions per 32 pairs where the exact test takes 165,000 cycles.
-// 4,001 closures: 35.0 -> 4.2 ms; 16,000: 556 -> 60 ms. Bound by FP32 issue
+// 3D, 4,001 closures: 35.0 -> 4.0 ms; 16,000: 556 -> 60 ms. 2D, 3,000 closures:
+// 5.3 -> 0.96 ms; 12,000: 80.7 -> 10.9 ms. Bound by FP32 issue
 // (about 0.6 of its rate); the rest is instruction fetch: the code is larger
 // than the first-level instruction cache, so the phases' loops are rolled (115
 // -> 63 ms) and the 12 warps of a block go through the phases together (-> 60
 // ms; with 4, 8 and 16 warps 64, 66 and 72 ms).
-// k_pair_filter3 leaves its verdicts in `lower` and its unsure pairs as bits in
-// `unsure` (both one word per 32 x 1 tile); k_pair_exact3 gathers those bits
+// k_pair_filter leaves its verdicts in `lower` and its unsure pairs as bits in
+// `unsure` (both one word per 32 x 1 tile); k_pair_exact gathers those bits
 // into full warps and adds the consistent ones to `lower`.
 
 // per-closure data of the filter: a thread per value, the last one the closure's premises
-__global__ void k_filter_pack3(int n, const int32_t* __restrict__ sa, const int32_t* __restrict__ sb,
-                               const double* __restrict__ zp, const double* __restrict__ zc, TrajView tr,
-                               pf::D2* __restrict__ df, float* __restrict__ f, uint8_t* __restrict__ ok) {
+template <int DIM>
+__global__ void k_filter_pack(int n, const int32_t* __restrict__ sa, const int32_t* __restrict__ sb,
+                              const double* __restrict__ zp, const double* __restrict__ zc, TrajView tr,
+                              pf::D2* __restrict__ df, float* __restrict__ f, uint8_t* __restrict__ ok) {
+  using F = pf::Filter<DIM>;
+  constexpr int st = Lie<DIM>::stride, dd = Lie<DIM>::d * Lie<DIM>::d;
   const int k = blockIdx.x * blockDim.x + threadIdx.x, v = blockIdx.y;
   if (k >= n) return;
   const size_t a = sa[k], b = sb[k];
-  const double *pa = tr.pose + a * 12, *pb = tr.pose + b * 12, *ca = tr.cov + a * 36, *cb = tr.cov + b * 36;
-  const double *z = zp + (size_t)k * 12, *c = zc + (size_t)k * 36;
-  if (v < pf::kPairs) {
-    df[(size_t)v * n + k] = pf::pack_pair(v, pa, ca, pb, cb, z);
-  } else if (v < pf::kPairs + pf::kFloats) {
-    f[(size_t)(v - pf::kPairs) * n + k] = pf::pack_float(v - pf::kPairs, pa, ca, pb, cb, z, c);
-  } else {
-    ok[k] = tr.rot[a] && tr.rot[b] && pf::cov_premise(ca, true) && pf::cov_premise(cb, true) &&
-            pf::cov_premise(c, false) && pf::pose_premise(pa) && pf::pose_premise(pb) && pf::pose_premise(z);
-  }
+  const double *pa = tr.pose + a * st, *pb = tr.pose + b * st, *ca = tr.cov + a * dd, *cb = tr.cov + b * dd;
+  const double *z = zp + (size_t)k * st, *c = zc + (size_t)k * dd;
+  if (v < F::pairs)
+    df[(size_t)v * n + k] = F::pair(v, pa, ca, pb, cb, z);
+  else if (v < F::pairs + F::floats)
+    f[(size_t)(v - F::pairs) * n + k] = F::single(v - F::pairs, pa, ca, pb, cb, z, c);
+  else
+    ok[k] = tr.rot[a] && tr.rot[b] && F::premise(pa, ca, pb, cb, z, c);
 }
 
 struct BlockSync {
   __device__ void operator()() const { __syncthreads(); }
 };
-template <int ROWS>
-__global__ void __launch_bounds__(32 * ROWS) k_pair_filter3(int n, int row_begin, const uint8_t* __restrict__ flip,
-                                                            pf::Group g, float th2, uint32_t* __restrict__ lower,
-                                                            uint32_t* __restrict__ unsure, int words) {
+template <int DIM, int ROWS>
+__global__ void __launch_bounds__(32 * ROWS) k_pair_filter(int n, int row_begin, const uint8_t* __restrict__ flip,
+                                                           pf::Group g, float th2, uint32_t* __restrict__ lower,
+                                                           uint32_t* __restrict__ unsure, int words) {
   const int lane = threadIdx.x;
   const int j0 = row_begin + ROWS * blockIdx.y, i0 = 32 * blockIdx.x;
   if (i0 >= min(j0 + ROWS, n) - 1) return;  // whole block: tiles above the diagonal
   const int j = min(j0 + (int)threadIdx.y, n - 1), i = min(i0 + lane, n - 1);
-  const int r = pf::verdict(g, i, j, flip[i] != flip[j], th2, BlockSync());
+  const int r = pf::Filter<DIM>::test(g, i, j, flip[i] != flip[j], th2, BlockSync());
   const bool pair = j0 + (int)threadIdx.y < n && i0 + lane < j;
   const unsigned yes = __ballot_sync(0xffffffffu, pair && r == 1), open = __ballot_sync(0xffffffffu, pair && r == 2);
   if (lane == 0 && j0 + (int)threadIdx.y < n && i0 < j) {
@@ -689,7 +691,8 @@ __global__ void __launch_bounds__(32 * ROWS) k_pair_filter3(int n, int row_begin
 constexpr int kExactThreads = 128;
 // each block takes `chunk` consecutive words of the rows x nb tiles: their set
 // bits go to a list in shared memory, which the block works off a full block at a time
-__global__ void __launch_bounds__(kExactThreads) k_pair_exact3(
+template <int DIM>
+__global__ void __launch_bounds__(kExactThreads) k_pair_exact(
     int n, int row_begin, int nb, int64_t chunk, const int32_t* __restrict__ sa, const int32_t* __restrict__ sb,
     const uint8_t* __restrict__ flip, const double* __restrict__ zp, const double* __restrict__ zc, TrajView tr,
     double th0, const uint32_t* __restrict__ unsure, uint32_t* __restrict__ lower, int words,
@@ -719,7 +722,7 @@ __global__ void __launch_bounds__(kExactThreads) k_pair_exact3(
       left -= take;
       if ((int)threadIdx.x < take) {
         const int2 p = list[left + threadIdx.x];
-        if (pair_consistent<3, PWC<3>>(p.x, p.y, sa, sb, flip, zp, zc, tr, th0, 0.0, pre))
+        if (pair_consistent<DIM, PWC<DIM>>(p.x, p.y, sa, sb, flip, zp, zc, tr, th0, 0.0, pre))
           atomicOr(lower + (size_t)(p.y - row_begin) * words + (p.x >> 5), 1u << (p.x & 31));
       }
     }
@@ -819,6 +822,41 @@ void launch_odom_check(int dim, int mode, int64_t count, const int32_t* si, cons
   RPGO_LAUNCHED();
 }
 
+namespace {
+struct PairFilter {
+  DeviceBuffer<pf::D2> df;
+  DeviceBuffer<float> f;
+  DeviceBuffer<uint8_t> ok;
+  DeviceBuffer<uint32_t> unsure;
+  void resize(int dim, int n, size_t tiles) {
+    df.resize((size_t)(dim == 3 ? pf::Filter<3>::pairs : pf::Filter<2>::pairs) * n);
+    f.resize((size_t)(dim == 3 ? pf::Filter<3>::floats : pf::Filter<2>::floats) * n);
+    ok.resize(n);
+    unsure.resize(tiles);
+  }
+};
+
+template <int DIM>
+void pair_filter(PairFilter& p, int n, int row_begin, const int32_t* sa, const int32_t* sb, const uint8_t* flip,
+                 const double* zp, const double* zc, TrajView tr, double th, uint32_t* lower, int words,
+                 const double* pre, cudaStream_t st) {
+  using F = pf::Filter<DIM>;
+  constexpr int FR = 12;
+  const int rows = n - row_begin;
+  k_filter_pack<DIM><<<dim3(div_up(n, 128), F::pairs + F::floats + 1), 128, 0, st>>>(
+      n, sa, sb, zp, zc, tr, p.df.get(), p.f.get(), p.ok.get());
+  RPGO_LAUNCHED();
+  const pf::Group g{p.df.get(), p.f.get(), p.ok.get(), n};
+  k_pair_filter<DIM, FR><<<dim3(div_up(n, 32), div_up(rows, FR)), dim3(32, FR), 0, st>>>(
+      n, row_begin, flip, g, (float)(th * th), lower, p.unsure.get(), words);
+  RPGO_LAUNCHED();
+  const int nb = div_up(n, 32), blocks = 4 * device_sm_count();
+  const int64_t chunk = std::max<int64_t>(kExactThreads, ((int64_t)rows * nb + blocks - 1) / blocks);
+  k_pair_exact<DIM><<<div_up((int64_t)rows * nb, chunk), kExactThreads, 0, st>>>(
+      n, row_begin, nb, chunk, sa, sb, flip, zp, zc, tr, th, p.unsure.get(), lower, words, pre);
+}
+}  // namespace
+
 void launch_pairwise(int dim, int mode, int n, int row_begin, const int32_t* sa, const int32_t* sb,
                      const uint8_t* flip, const double* zp, const double* zc, TrajView tr, double th0, double th1,
                      uint32_t* adj, int words, uint32_t* lower_scratch, cudaStream_t st) {
@@ -836,33 +874,17 @@ void launch_pairwise(int dim, int mode, int n, int row_begin, const int32_t* sa,
     // The filter and the exact test of what it leaves take two launches, and
     // the second lasts at least one exact test (90 us) where it has any pair:
     // below 65,536 pairs, which the exact test alone takes in three waves,
-    // they are not faster.
+    // they are not faster. (2D, exact alone and with the filter: 363 closures,
+    // 65,703 pairs, 0.30 and 0.28 ms with the transfers; 1,000: 0.79 and 0.35.)
     const double pairs = 0.5 * n * (n - 1.0) - 0.5 * row_begin * (row_begin - 1.0);
-    const bool filter = dim == 3 && mode == 0 && pairs >= 65536.0 && th0 > 0.0 && th0 < 1e15;
-    DeviceBuffer<pf::D2> fdf;
-    DeviceBuffer<float> ff;
-    DeviceBuffer<uint8_t> fok;
-    DeviceBuffer<uint32_t> unsure;
-    if (filter) {
-      fdf.resize((size_t)pf::kPairs * n);
-      ff.resize((size_t)pf::kFloats * n);
-      fok.resize(n);
-      unsure.resize((size_t)rows * words);
-    }
+    const bool filter = mode == 0 && pairs >= 65536.0 && th0 > 0.0 && th0 < 1e15;
+    PairFilter pack;
+    if (filter) pack.resize(dim, n, (size_t)rows * words);
     EventTimer timer(st);
-    if (filter) {
-      k_filter_pack3<<<dim3(div_up(n, 128), pf::kPairs + pf::kFloats + 1), 128, 0, st>>>(
-          n, sa, sb, zp, zc, tr, fdf.get(), ff.get(), fok.get());
-      RPGO_LAUNCHED();
-      constexpr int FR = 12;
-      const pf::Group g{fdf.get(), ff.get(), fok.get(), n};
-      k_pair_filter3<FR><<<dim3(div_up(n, 32), div_up(rows, FR)), dim3(32, FR), 0, st>>>(
-          n, row_begin, flip, g, (float)(th0 * th0), lower_scratch, unsure.get(), words);
-      RPGO_LAUNCHED();
-      const int nb = div_up(n, 32), blocks = 4 * device_sm_count();
-      const int64_t chunk = std::max<int64_t>(kExactThreads, ((int64_t)rows * nb + blocks - 1) / blocks);
-      k_pair_exact3<<<div_up((int64_t)rows * nb, chunk), kExactThreads, 0, st>>>(
-          n, row_begin, nb, chunk, sa, sb, flip, zp, zc, tr, th0, unsure.get(), lower_scratch, words, pre.get());
+    if (filter && dim == 3) {
+      pair_filter<3>(pack, n, row_begin, sa, sb, flip, zp, zc, tr, th0, lower_scratch, words, pre.get(), st);
+    } else if (filter) {
+      pair_filter<2>(pack, n, row_begin, sa, sb, flip, zp, zc, tr, th0, lower_scratch, words, nullptr, st);
     } else if (dim == 3) {
       if (mode == 0)
         k_pairwise<3, PWC<3>, ROWS><<<grid, block, 0, st>>>(n, row_begin, sa, sb, flip, zp, zc, tr, th0, th1,

@@ -5,25 +5,37 @@
 
 #include "pcm_filter.cuh"
 
-extern "C" {
+namespace {
 
-// out[j * n + i], i < j: 0 inconsistent, 1 consistent, 2 unsure
-void pair_filter(int n, const int32_t* sa, const int32_t* sb, const uint8_t* flip, const double* zp,
-                 const double* zc, const double* tp, const double* tc, const uint8_t* rot, double th, uint8_t* out) {
+template <int DIM>
+void run(int n, const int32_t* sa, const int32_t* sb, const uint8_t* flip, const double* zp, const double* zc,
+         const double* tp, const double* tc, const uint8_t* rot, double th, uint8_t* out) {
   using namespace rpgo::pf;
-  std::vector<D2> df((size_t)kPairs * n);
-  std::vector<float> f((size_t)kFloats * n);
+  using F = Filter<DIM>;
+  constexpr int st = DIM == 3 ? 12 : 4, dd = DIM == 3 ? 36 : 9;
+  std::vector<D2> df((size_t)F::pairs * n);
+  std::vector<float> f((size_t)F::floats * n);
   std::vector<uint8_t> ok(n);
   for (int k = 0; k < n; ++k) {
-    const double *pa = tp + 12 * sa[k], *pb = tp + 12 * sb[k], *ca = tc + 36 * sa[k], *cb = tc + 36 * sb[k];
-    const double *z = zp + 12 * k, *c = zc + 36 * k;
-    for (int v = 0; v < kPairs; ++v) df[(size_t)v * n + k] = pack_pair(v, pa, ca, pb, cb, z);
-    for (int v = 0; v < kFloats; ++v) f[(size_t)v * n + k] = pack_float(v, pa, ca, pb, cb, z, c);
-    ok[k] = rot[sa[k]] && rot[sb[k]] && cov_premise(ca, true) && cov_premise(cb, true) && cov_premise(c, false) &&
-            pose_premise(pa) && pose_premise(pb) && pose_premise(z);
+    const double *pa = tp + st * sa[k], *pb = tp + st * sb[k], *ca = tc + dd * sa[k], *cb = tc + dd * sb[k];
+    const double *z = zp + st * k, *c = zc + dd * k;
+    for (int v = 0; v < F::pairs; ++v) df[(size_t)v * n + k] = F::pair(v, pa, ca, pb, cb, z);
+    for (int v = 0; v < F::floats; ++v) f[(size_t)v * n + k] = F::single(v, pa, ca, pb, cb, z, c);
+    ok[k] = rot[sa[k]] && rot[sb[k]] && F::premise(pa, ca, pb, cb, z, c);
   }
   const Group g{df.data(), f.data(), ok.data(), n};
   for (int j = 0; j < n; ++j)
-    for (int i = 0; i < j; ++i) out[(size_t)j * n + i] = (uint8_t)verdict(g, i, j, flip[i] != flip[j], (float)(th * th));
+    for (int i = 0; i < j; ++i) out[(size_t)j * n + i] = (uint8_t)F::test(g, i, j, flip[i] != flip[j], (float)(th * th));
+}
+
+}  // namespace
+
+extern "C" {
+
+// out[j * n + i], i < j: 0 inconsistent, 1 consistent, 2 unsure
+void pair_filter(int dim, int n, const int32_t* sa, const int32_t* sb, const uint8_t* flip, const double* zp,
+                 const double* zc, const double* tp, const double* tc, const uint8_t* rot, double th, uint8_t* out) {
+  if (dim == 3) run<3>(n, sa, sb, flip, zp, zc, tp, tc, rot, th, out);
+  else run<2>(n, sa, sb, flip, zp, zc, tp, tc, rot, th, out);
 }
 }

@@ -7,7 +7,7 @@ import pytest
 
 from oracle import rpgo_oracle as O
 from rpgo_gb300 import capi
-from test_pair_filter_cpu import group
+from test_pair_filter_cpu import exact, group, group2
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +67,24 @@ def test_new_rows_and_stride(closures, row_begin, extra):
         assert rc == 0
     got = adj.cpu().numpy().view(np.uint32)[:, :want.shape[1]]
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [362, 363, 385, 700])
+@pytest.mark.parametrize("th", [5.0, 0.4])
+def test_adjacency_is_the_oracles_2d(n, th):
+    g = group2(3000, 520, 240, 3)
+    rng = np.random.default_rng(6)
+    m = len(g["sa"])
+    assert m >= 700
+    g["flip"] = (rng.random(m) < 0.2).astype(np.uint8)
+    for k in rng.choice(m, 8, replace=False):
+        g["zc"][k][0, 0] = np.nan
+    for k in rng.choice(m, 6, replace=False):
+        g["sb"][k] = g["sa"][k]
+    for s in rng.choice(3000, 30, replace=False):
+        g["rot"][s] = 0
+    g = _cut(g, n)
+    got = capi.pairwise_adjacency(2, 0, g["sa"], g["sb"], g["flip"], g["z"], g["zc"], g["pose"], g["cov"],
+                                  np.zeros(len(g["rot"]), np.int32), g["rot"], th, 0.0)
+    got = np.unpackbits(np.asarray(got).view(np.uint8).reshape(n, -1), axis=1, bitorder="little")[:, :n]
+    assert np.array_equal(got, exact(g, th))
