@@ -6,7 +6,8 @@
 // / GaussNewtonParams built in src/RobustSolver.cpp:120-300 keep GTSAM's
 // default linearSolverType). Here the same system is factored on the GPU.
 // The plan fixes, once per graph structure:
-//  * an elimination order (minimum degree on the pose graph, ties by index);
+//  * an elimination order (the cheaper of minimum degree, with the elimination
+//    tree's level counted in on smaller graphs, and two nested dissections);
 //  * the block structure of L and its elimination tree;
 //  * a split into sparse columns, scheduled by elimination-tree level, and a
 //    trailing dense block (the columns whose structure is already complete);
