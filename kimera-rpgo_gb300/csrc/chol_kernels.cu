@@ -1108,7 +1108,10 @@ struct DfSmem {
   double X[kTB][kTB + 1];             // the dense tail
 };
 
-__device__ __forceinline__ void df_mat_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kDfMat) : "memory"); }
+__device__ __forceinline__ void df_mat_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(kDfMat) : "memory");
+}
 
 // v > 0 (false for NaN), from its bits: an FP64 comparison costs 64 cycles
 __device__ __forceinline__ bool positive(double v) {
@@ -1138,6 +1141,7 @@ __device__ __forceinline__ void df_factor(const CholArgs& a, int j, int lane, Df
       v = r == k ? il : v * il;
       if (lane < ntri) s.Lj[r * D + c] = v;
     }
+    __syncwarp();
     asm volatile("bar.arrive %0, %1;" ::"r"(kPivotBar + k), "n"(kDfMat) : "memory");
     if (k + 1 < D) {
       const double lr = __shfl_sync(kFull, v, r >= k ? r * (r + 1) / 2 + k : 0);
@@ -1238,6 +1242,7 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
         double v = on ? s.S[dd + rr * D + r] : 0.0;
 #pragma unroll
         for (int c = 0; c < D; ++c) {
+          __syncwarp();
           if (rr0 == 0) asm volatile("bar.sync %0, %1;" ::"r"(kPivotBar + c), "n"(kDfMat) : "memory");
           const double x = __shfl_sync(kFull, v, base + c) * s.Lj[c * D + c];
           if (r == c) v = x;
@@ -1297,46 +1302,47 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
   double* yt = a.y + (size_t)a.ns * D;
   double b = 0.0;  // warp 7: the right-hand side, a row per lane
   if (wi < kDfMat / 32) {
-    const int ni = a.T * (a.T + 1) / 2 * dd;
-    for (int i0 = 0; i0 < ni; i0 += kDfMat) {
-      const int it = i0 + threadIdx.x, t = it / dd, e = it % dd, rr = e / D, cc = e % D;
-      const bool on = it < ni;
-      int bi = 0, bj = on ? t : 0;
-      while (bj > bi) bj -= ++bi;
-      const int2 bl = on ? reinterpret_cast<const int2*>(a.df_blk)[a.df_tail_blk + t] : make_int2(0, 0);
-      double v = 0.0;
-      if (on)
-        v = bi == bj ? gather_diag<D>(a, a.perm[a.ns + bi], rr, cc)
-                     : gather_offdiag<D>(a.fH64, a.ta_src, a.ta_ptr[t], a.ta_ptr[t + 1], rr, cc);
-      constexpr int W = 8;
-      const int np = __reduce_max_sync(kFull, bl.y);
-      for (int u = 0; u < np; u += W)
-        add_words<W, 1>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, false, v);
-      __syncwarp();
-      if (on) s.X[bi * D + rr][bj * D + cc] = v;
-    }
+    // (tail_fits: an entry of the blocks per thread)
+    const int it = threadIdx.x, b_it = it / dd, e = it % dd, rr = e / D, cc = e % D;
+    const bool on = it < a.T * (a.T + 1) / 2 * dd;
+    int bi = 0, bj = on ? b_it : 0;
+    while (bj > bi) bj -= ++bi;
+    const int2 bl = on ? reinterpret_cast<const int2*>(a.df_blk)[a.df_tail_blk + b_it] : make_int2(0, 0);
+    double v = 0.0;
+    if (on)
+      v = bi == bj ? gather_diag<D>(a, a.perm[a.ns + bi], rr, cc)
+                   : gather_offdiag<D>(a.fH64, a.ta_src, a.ta_ptr[b_it], a.ta_ptr[b_it + 1], rr, cc);
+    constexpr int W = 8;
+    const int np = __reduce_max_sync(kFull, bl.y);
+    for (int u = 0; u < np; u += W)
+      add_words<W, 1>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, false, v);
+    __syncwarp();
+    if (on) s.X[bi * D + rr][bj * D + cc] = v;
+    __syncwarp();
     df_mat_sync();
     // Right-looking, one column per step: warp 0 (a row per lane) scales
     // column c and brings column c + 1 up to date by itself, so that its next
     // pivot does not wait for the block; the other warps subtract column c
     // from the columns behind, an entry per thread.
-    constexpr int kOthers = kDfMat - 32;
-    int er[2], eq[2];
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      int e = (int)threadIdx.x - 32 + x * kOthers;
-      er[x] = eq[x] = 0;
-      if (wi > 0 && e < n * (n + 1) / 2) {
-        while (e > er[x]) e -= ++er[x];
-        eq[x] = e;
-      }
+    int er = 0, eq = 0;
+    if (wi > 0 && (int)threadIdx.x - 32 < n * (n + 1) / 2) {
+      int e = (int)threadIdx.x - 32;
+      while (e > er) e -= ++er;
+      eq = e;
     }
     // Named barriers: 3 publishes column c (warp 0 arrives, the others wait),
     // 4 and 5 in turn say that the others are done with it (they arrive, warp 0
     // waits one step later; it arrives at 3 for column c + 1 before that, so the
-    // others can be one step ahead of its wait, and no more).
-    auto wait = [](int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDfMat) : "memory"); };
-    auto arrive = [](int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kDfMat) : "memory"); };
+    // others can be one step ahead of its wait, and no more). A warp has to be
+    // converged at each.
+    auto wait = [](int id) {
+      __syncwarp();
+      asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
+    };
+    auto arrive = [](int id) {
+      __syncwarp();
+      asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
+    };
     if (wi == 0) {
       double col = lane < n ? s.X[lane][0] : 0.0;
       for (int c = 0; c < n; ++c) {
@@ -1356,9 +1362,7 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
     } else {
       for (int c = 0; c < n; ++c) {
         wait(3);
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (eq[x] > c + 1) s.X[er[x]][eq[x]] = fma(-s.X[er[x]][c], s.X[eq[x]][c], s.X[er[x]][eq[x]]);
+        if (eq > c + 1) s.X[er][eq] = fma(-s.X[er][c], s.X[eq][c], s.X[er][eq]);
         arrive(4 + (c & 1));
       }
     }

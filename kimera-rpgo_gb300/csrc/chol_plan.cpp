@@ -880,7 +880,7 @@ void add_dataflow(CholPlan& p, int max_cols) {
   const int w0 = p.lvl_col_ptr[l0];
   std::vector<uint8_t> in_df(ns, 0);
   for (int w = w0; w < ns; ++w) in_df[p.lvl_cols[w]] = 1;
-  p.df_tail = p.n_tiles <= 1;
+  p.df_tail = tail_fits(p.T, p.d);
   for (int t = 0; t < p.n_tail_blocks() && p.df_tail; ++t)
     if (p.tupd_ptr[t + 1] - p.tupd_ptr[t] > tail_slots(p.d)) p.df_tail = 0;
   // products and rows of the part's columns, then of the tail

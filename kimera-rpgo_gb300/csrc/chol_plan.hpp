@@ -26,6 +26,11 @@ constexpr int kDfMaxBlocks = 15, kDfMaxChunks = 64, kDfColInts = 8;
 // lane groups of a CTA of the solve kernel: the dense tail's blocks add their
 // update pairs in this many interleaved chains
 constexpr int tail_slots(int d) { return 8 * (32 / d); }
+// the dense tail's blocks, and the lower triangle of their scalars, fit one
+// entry per thread of the warps that assemble (7) and update (6) them
+constexpr bool tail_fits(int T, int d) {
+  return T * (T + 1) / 2 * d * d <= 7 * 32 && T * d * (T * d + 1) / 2 <= 6 * 32;
+}
 
 struct CholPlan {
   int N = 0;             // variables (block columns)
@@ -82,8 +87,7 @@ struct CholPlan {
   // update pair whose target block is in such a column (the block's first
   // pair carries the Hessian block) or, with df_tail set, in the dense tail;
   // the products of a block are numbered consecutively in pair order. df_tail:
-  // the tail has at most one tile and none of its blocks more pairs than
-  // tail_slots.
+  // tail_fits, and none of the tail's blocks has more pairs than tail_slots.
   //  df_col: kDfColInts ints per column: position, first block, off-diagonal
   //    blocks m, first entry of df_blk, first entry of df_dst, first entry of
   //    df_row, entries of df_row, 0;

@@ -39,7 +39,7 @@ int check(const CholPlan& p, int max_cols) {
     const int j = r[0], p0 = r[1], m = r[2];
     if (j != p.lvl_cols[w0 + w] || p0 != p.col_ptr[j] || m != p.col_ptr[j + 1] - p0 - 1) return 5;
     if (m > rpgo::kDfMaxBlocks) return 6;
-    const int32_t* d = &p.df_dst[(size_t)4 * r[4]];
+    const int32_t* d = p.df_dst.data() + (size_t)4 * r[4];
     for (int a = 0; a < m; ++a)
       for (int b = a; b < m; ++b, d += 4) {
         if (d[2] != a || d[3] != b) return 7;
@@ -77,7 +77,7 @@ int check(const CholPlan& p, int max_cols) {
       np += p.upd_ptr[q + 1] - p.upd_ptr[q];
     }
   }
-  bool tail = p.n_tiles <= 1;
+  bool tail = rpgo::tail_fits(p.T, p.d);
   for (int t = 0; t < p.n_tail_blocks(); ++t)
     tail = tail && p.tupd_ptr[t + 1] - p.tupd_ptr[t] <= rpgo::tail_slots(p.d);
   if ((p.df_tail != 0) != tail) return 15;

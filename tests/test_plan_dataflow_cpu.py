@@ -32,6 +32,8 @@ def _graph(shape, n, seed):
         return chain
     if shape == "near":
         return chain + [(i, min(n - 1, i + int(rng.integers(2, 9)))) for i in rng.integers(0, max(n - 3, 1), n // 4)]
+    if shape == "tail4":  # a dense tail of four blocks: 24 scalars at d = 6, more entries than threads
+        return chain + [(38, 49), (28, 39), (33, 27)]
     if shape == "far":
         return chain + [tuple(int(x) for x in rng.choice(n, 2, replace=False)) for _ in range(n // 5)]
     return chain + [(0, i) for i in range(2, n)]  # a hub: columns beyond the part's limits
@@ -39,7 +41,7 @@ def _graph(shape, n, seed):
 
 @pytest.mark.parametrize("d", [3, 6])
 @pytest.mark.parametrize("shape,n", [("alone", 1), ("alone", 5), ("chain", 2), ("chain", 3), ("chain", 70),
-                                     ("near", 40), ("near", 700), ("far", 60), ("far", 400), ("hub", 60)])
+                                     ("near", 40), ("near", 700), ("tail4", 50), ("far", 60), ("far", 400), ("hub", 60)])
 @pytest.mark.parametrize("cols", [0, 1, 7, 60, 1216])
 def test_dataflow_lists_match_the_level_form(lib, d, shape, n, cols):
     e = _graph(shape, n, n)
