@@ -1033,12 +1033,13 @@ __device__ void tail_backward_item(const CholArgs& a, double* yt, int k, TileSme
 // df_stall, on which all waits end, and the host reports the solve as failed.
 // Waits are warp-wide: lanes that left a wait one by one would issue the
 // FP64 work behind it one by one (64 cycles each time).
-// Bound by the FP64 chain of a column (about 8,500 cycles from one level to
-// the next: six reciprocal square roots, 3,800 of them in all with their
-// products and FMAs, the row solves 1,400, the products 800, the hand-over
-// and the sums). Per solve, level form before -> now: 300 poses 264 -> 122
-// us, 5,000 poses 397 -> 214, 20,000 poses 617 -> 402, 50,000 poses 1,017 ->
-// 780.
+// Bound by the FP64 chain of a column (about 6,700 cycles from one level to
+// the next at 300 poses: six reciprocal square roots with their products and
+// FMAs 3,800, then what is left of the row solves, the products, the hand-over
+// and the sums). Per solve, level form before -> now in the same order of
+// elimination: 300 poses 264 -> 111 us, a 2D walk of 500 199 -> 79, 5,000 poses
+// 397 -> 208, 20,000 617 -> 402, 50,000 1,017 -> 780 (and 73 and 57 us for the
+// first two in the order by level of chol_plan.cpp).
 constexpr unsigned long long kEmpty = 0x7ffcd5c3a19b42e7ull;  // a NaN that no operation produces
 constexpr int kDfSpins = 1 << 21;
 constexpr int kPivotBar = 3;           // named barriers 3 .. 3 + D - 1: a column of L_jj is in place
@@ -1290,7 +1291,7 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
   __syncthreads();  // s is reused by the CTA's next column
 }
 
-// The dense tail of one tile by one CTA, with the order of tail_block_cta,
+// A dense tail of tail_fits by one CTA, with the order of tail_block_cta,
 // smem_chol and the two substitutions: its blocks' products are added as
 // they arrive, so the phases and barriers that assembled, factored and
 // solved it after the last column (30 us) shrink to the factorisation.
@@ -1793,8 +1794,8 @@ __global__ void __launch_bounds__(kThreads) k_chol_solve(CholArgs a) {
 }
 
 // The assembly, in one launch (it took two, and the second one read back what
-// the first had just written: 16 -> 9 us at 300 poses). The first var_blocks
-// blocks take a warp per variable: lane e owns entries e and e + 32 of its
+// the first had just written: 17 -> 9 us at 300 poses, cold caches). The first
+// var_blocks blocks take a warp per variable: lane e owns entries e and e + 32 of its
 // diagonal block (and gradient entry e < D), summed over its factors in their
 // order; written per variable and, with the damping diagonal, in the factor's
 // block layout. The others take a thread per row of an off-diagonal block,

@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(128) k_linearize_a(int F, const int32_t* __res
   // then forms the adjoint and the whitened residual; the role-1 warp forms
   // the log-map Jacobian. With res the log map and the relative pose are those
   // that the error sum at the same values has left there (the same operations,
-  // so the same bits); without (joint batches), role 0 evaluates them: 22 -> 14
-  // us a pass at 300 poses.
+  // so the same bits); without (joint batches), role 0 evaluates them: 23 -> 15
+  // us a pass at 300 poses, 22 -> 14 at 5,000 (cold caches).
   __shared__ double sh_e[2][32][d];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = warp >> 1, role = warp & 1;
