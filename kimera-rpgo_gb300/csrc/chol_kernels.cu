@@ -41,6 +41,7 @@
 #include <cooperative_groups.h>
 
 #include "chol.hpp"
+#include "tail_barriers.hpp"
 
 namespace cg = cooperative_groups;
 
@@ -1029,8 +1030,11 @@ __device__ void tail_backward_item(const CholArgs& a, double* yt, int k, TileSme
 // form (chunk by chunk), so the factor has the same bits.
 // Columns are taken in level order by CTAs that are all resident
 // (cooperative launch), so the lowest unfinished column never waits for one
-// that has no CTA. Every wait is bounded: after kDfSpins polls a CTA raises
-// df_stall, on which all waits end, and the host reports the solve as failed.
+// that has no CTA. Every wait for a word is bounded: after kDfSpins polls a CTA
+// raises df_stall, on which all of them end, and the host reports the solve as
+// failed. The waits at named barriers have no limit of their own; they end
+// because every warp of the CTA comes to each of them, in an order that does
+// not depend on data (the tail's: tail_barriers.hpp).
 // Waits are warp-wide: lanes that left a wait one by one would issue the
 // FP64 work behind it one by one (64 cycles each time).
 // Bound by the FP64 chain of a column (about 6,700 cycles from one level to
@@ -1291,6 +1295,18 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
   __syncthreads();  // s is reused by the CTA's next column
 }
 
+// named barriers of the warps that work on the column's or tail's blocks
+struct TailBarriers {
+  __device__ __forceinline__ void wait(int id) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
+  }
+  __device__ __forceinline__ void arrive(int id) {
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
+  }
+};
+
 // A dense tail of tail_fits by one CTA, with the order of tail_block_cta,
 // smem_chol and the two substitutions: its blocks' products are added as
 // they arrive, so the phases and barriers that assembled, factored and
@@ -1331,41 +1347,29 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
       while (e > er) e -= ++er;
       eq = e;
     }
-    // Named barriers: 3 publishes column c (warp 0 arrives, the others wait),
-    // 4 and 5 in turn say that the others are done with it (they arrive, warp 0
-    // waits one step later; it arrives at 3 for column c + 1 before that, so the
-    // others can be one step ahead of its wait, and no more). A warp has to be
-    // converged at each.
-    auto wait = [](int id) {
-      __syncwarp();
-      asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
-    };
-    auto arrive = [](int id) {
-      __syncwarp();
-      asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
-    };
+    // (the order of the barriers, and why it ends: tail_barriers.hpp)
+    TailBarriers bar;
     if (wi == 0) {
-      double col = lane < n ? s.X[lane][0] : 0.0;
-      for (int c = 0; c < n; ++c) {
-        const double piv = __shfl_sync(kFull, col, c);
-        const bool pos = positive(piv);
-        const double il = rsqrt(pos ? piv : 1.0);
-        if (!pos && lane == 0) set_fail(a.status);
-        const double l = lane == c ? il : col * il;
-        if (lane >= c && lane < n) s.X[lane][c] = l;
-        arrive(3);
-        if (c > 0) wait(4 + ((c - 1) & 1));
-        // column c + 1: the others have subtracted columns 0 .. c - 1 from it
-        const double lq = __shfl_sync(kFull, l, min(c + 1, n - 1));
-        if (lane > c && lane < n && c + 1 < n) col = fma(-l, lq, s.X[lane][c + 1]);
-      }
-      wait(4 + ((n - 1) & 1));
+      double col = lane < n ? s.X[lane][0] : 0.0, l = 0.0;
+      tail_lead(
+          n, bar,
+          [&](int c) {
+            const double piv = __shfl_sync(kFull, col, c);
+            const bool pos = positive(piv);
+            const double il = rsqrt(pos ? piv : 1.0);
+            if (!pos && lane == 0) set_fail(a.status);
+            l = lane == c ? il : col * il;
+            if (lane >= c && lane < n) s.X[lane][c] = l;
+          },
+          [&](int c) {
+            // column c + 1: the others have subtracted columns 0 .. c - 1 from it
+            const double lq = __shfl_sync(kFull, l, min(c + 1, n - 1));
+            if (lane > c && lane < n && c + 1 < n) col = fma(-l, lq, s.X[lane][c + 1]);
+          });
     } else {
-      for (int c = 0; c < n; ++c) {
-        wait(3);
+      tail_follow(n, bar, [&](int c) {
         if (eq > c + 1) s.X[er][eq] = fma(-s.X[er][c], s.X[eq][c], s.X[er][eq]);
-        arrive(4 + (c & 1));
-      }
+      });
     }
   } else {
     for (int t = 0; t < a.T; ++t) {
