@@ -426,7 +426,18 @@ __device__ void column_warp(const CholArgs& a, int j, int lane) {
   forward_solve<D>(a, j, g == 0, r, base, C, forward_rhs<D>(a, j, r));
 }
 
-__device__ __forceinline__ void team_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+// Named barriers of `threads` threads. Both take the warp as a whole (bar is
+// the aligned form): lanes that left a branch or a loop before them on their
+// own would come to them one by one, so each starts with a warp barrier.
+__device__ __forceinline__ void bar_wait(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void team_sync(int id) { bar_wait(id, 64); }
 
 // phase B for column j by a team of two warps (tw 0 = lead, 1 = helper) that
 // meet at named barrier `bar`; sh = D x D + D doubles of shared memory. The
@@ -1113,10 +1124,7 @@ struct DfSmem {
   double X[kTB][kTB + 1];             // the dense tail
 };
 
-__device__ __forceinline__ void df_mat_sync() {
-  __syncwarp();
-  asm volatile("bar.sync 1, %0;" ::"n"(kDfMat) : "memory");
-}
+__device__ __forceinline__ void df_mat_sync() { bar_wait(1, kDfMat); }
 
 // v > 0 (false for NaN), from its bits: an FP64 comparison costs 64 cycles
 __device__ __forceinline__ bool positive(double v) {
@@ -1146,8 +1154,7 @@ __device__ __forceinline__ void df_factor(const CholArgs& a, int j, int lane, Df
       v = r == k ? il : v * il;
       if (lane < ntri) s.Lj[r * D + c] = v;
     }
-    __syncwarp();
-    asm volatile("bar.arrive %0, %1;" ::"r"(kPivotBar + k), "n"(kDfMat) : "memory");
+    bar_arrive(kPivotBar + k, kDfMat);
     if (k + 1 < D) {
       const double lr = __shfl_sync(kFull, v, r >= k ? r * (r + 1) / 2 + k : 0);
       const double lc = __shfl_sync(kFull, v, c >= k ? c * (c + 1) / 2 + k : 0);
@@ -1239,7 +1246,7 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
     // the solve is left after the last pivot.
     if (wi == 0) {
       df_factor<D>(a, j, lane, s);
-      asm volatile("bar.arrive 2, 64;" ::: "memory");  // L_jj for the right-hand side's warp
+      bar_arrive(2, 64);  // L_jj for the right-hand side's warp
     } else {
       for (int rr0 = 0; rr0 == 0 || rr0 < m * D; rr0 += (kDfMat / 32 - 1) * G) {
         const int rr = rr0 + (wi - 1) * G + g;
@@ -1248,7 +1255,7 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
 #pragma unroll
         for (int c = 0; c < D; ++c) {
           __syncwarp();
-          if (rr0 == 0) asm volatile("bar.sync %0, %1;" ::"r"(kPivotBar + c), "n"(kDfMat) : "memory");
+          if (rr0 == 0) bar_wait(kPivotBar + c, kDfMat);
           const double x = __shfl_sync(kFull, v, base + c) * s.Lj[c * D + c];
           if (r == c) v = x;
           else if (r > c) v = fma(-x, s.Lj[r * D + c], v);
@@ -1276,7 +1283,7 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
     // right-hand side: the row sums, then y_j
     const double sum = df_row_sum<D>(a, r1.y, r1.z, lane);
     double b = a.y[(size_t)j * D + r] - sum;
-    asm volatile("bar.sync 2, 64;" ::: "memory");
+    bar_wait(2, 64);
     double C[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) C[c] = c <= r ? s.Lj[r * D + c] : 0.0;
@@ -1297,14 +1304,8 @@ __device__ void df_column(const CholArgs& a, int w, DfSmem<D>& s) {
 
 // named barriers of the warps that work on the column's or tail's blocks
 struct TailBarriers {
-  __device__ __forceinline__ void wait(int id) {
-    __syncwarp();
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
-  }
-  __device__ __forceinline__ void arrive(int id) {
-    __syncwarp();
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kDfMat) : "memory");
-  }
+  __device__ __forceinline__ void wait(int id) { bar_wait(id, kDfMat); }
+  __device__ __forceinline__ void arrive(int id) { bar_arrive(id, kDfMat); }
 };
 
 // A dense tail of tail_fits by one CTA, with the order of tail_block_cta,
@@ -1335,7 +1336,6 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
       add_words<W, 1>(a, a.prod + (size_t)(bl.x + u) * dd + e, dd, bl.y - u, false, v);
     __syncwarp();
     if (on) s.X[bi * D + rr][bj * D + cc] = v;
-    __syncwarp();
     df_mat_sync();
     // Right-looking, one column per step: warp 0 (a row per lane) scales
     // column c and brings column c + 1 up to date by itself, so that its next

@@ -270,7 +270,9 @@ __global__ void __launch_bounds__(128) k_linearize_a(int F, const int32_t* __res
     }
 #pragma unroll
     for (int i = 0; i < d; ++i) sh_e[pair][lane][i] = e[i];
-    // (named barrier 1 + pair of the warp pair: role 0 arrives, role 1 waits)
+    // (named barrier 1 + pair of the warp pair: role 0 arrives, role 1 waits;
+    // both take the warp as a whole)
+    __syncwarp();
     asm volatile("bar.arrive %0, 64;" ::"r"(1 + pair) : "memory");
     if (!valid) return;
     if (between) {
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(128) k_linearize_a(int F, const int32_t* __res
     }
     out[d + 2 * dd] = sw;
   } else {
+    __syncwarp();
     asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
     if (!between) return;
     double e[d], D[dd];
