@@ -88,6 +88,16 @@ RPGO_HD float fabsv(float a) { return a < 0.f ? -a : a; }  // (NaN stays NaN)
 constexpr float kU = 5.9604644775390625e-8f;      // 2^-24
 constexpr float kDf = 3.637978807091713e-12f;     // 2^-38: about 2.4 times the worst case of a `between`
                                                   // (about 420 roundings of 2^-48)
+// A difference of two positions has an error of at most kDt (|t_a| + |t_c|)
+// (1-norms): 2^-48 of each from its pair, 2^-46 from the subtraction in pairs.
+// It moves the covariances through their lever arms: by kDt (|t_a| + |t_c|)
+// times what the lever's length multiplies. With the lever's magnitude written as
+// u + kLever (|t_a| + |t_c|), u the difference itself, half of kDf q_i q_j covers
+// it (kDf's own roundings take 1 / 2.4); in compositions in FP32, 4 of the 64
+// units of decide(), of which the roundings take 58.
+constexpr float kDt = 2.842170943040401e-14f;         // 2^-45
+constexpr float kLever = 0.015625f;                   // 2 kDt / kDf
+constexpr float kLeverFp32 = 1.1920928955078125e-7f;  // 2^22 kDt
 
 // ------------------------------------------------------------------ FP32 pairs
 struct alignas(8) D2 {
@@ -155,7 +165,8 @@ RPGO_HD float lo(D2 a) { return a.h; }
 // the closures of a group: value v of closure k is at [v * n + k].
 constexpr int kPairs = 78;   // FP32 pairs: pose a (R, t), cov a (lower), pose b, cov b, measured pose
 constexpr int kFloats = 44;  // FP32: inverse measurement's t (3), its covariance (21), sqrt of its diagonal (6),
-                             // sqrt of the diagonals of cov a and cov b (6 each), |t_a|, |t_b| (1-norms)
+                             // sqrt of the diagonals of cov a and cov b (6 each), |t_a|, |t_b| (1-norms, from the
+                             // group's origins)
 constexpr int kPoseA = 0, kCovA = 12, kPoseB = 33, kCovB = 45, kPoseZ = 66;
 constexpr int kZt = 0, kZc = 3, kZg = 24, kGA = 30, kGB = 36, kTA = 42, kTB1 = 43;
 RPGO_HD constexpr int tri(int i, int j) { return i * (i + 1) / 2 + j; }  // j <= i
@@ -180,25 +191,42 @@ struct Item {
 };
 RPGO_HD Item item(const Group& g, int k) { return Item{g.df + k, g.f + k, g.n}; }
 
+// Where a group's poses are measured from. A verdict depends on differences
+// of positions only, so the bounds need not grow with the distance of the map
+// from its frame's origin (a new robot's first pose can be anywhere, in metres
+// of a map grid for instance). A pair compares entries of one side of closure 0
+// with each other: the side of a closure that lies on side a (b) of closure 0
+// is measured from that endpoint of closure 0, flipped closures the other way
+// round. The subtraction is the one rounding that this adds, 2^-53 of the
+// result.
+struct Origin {
+  const double *a, *b;  // the poses whose positions endpoints a and b are measured from; null: the frame's
+};
+RPGO_HD double from_origin(double x, const double* origin, int at) {
+  if (!origin) return x;
+  const double o = origin[at];
+  return std::fabs(o) < 1e12 ? x - o : x;  // (NaN: as it is)
+}
 // value v of a closure from its trajectory entries (pose 12, covariance 36)
 // and measurement (pose 12)
 RPGO_HD D2 pack_pair(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                     const double* zp) {
-  if (v < kCovA) return split(pa[v]);
+                     const double* zp, Origin o = {nullptr, nullptr}) {
+  if (v < kCovA) return split(v < 9 ? pa[v] : from_origin(pa[v], o.a, v));
   if (v < kPoseB) return split(ca[tri_full(v - kCovA)]);
-  if (v < kCovB) return split(pb[v - kPoseB]);
+  if (v < kCovB) return split(v < kPoseB + 9 ? pb[v - kPoseB] : from_origin(pb[v - kPoseB], o.b, v - kPoseB));
   if (v < kPoseZ) return split(cb[tri_full(v - kCovB)]);
   return split(zp[v - kPoseZ]);
 }
 RPGO_HD float pack_float(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                         const double* zp, const double* zc) {
+                         const double* zp, const double* zc, Origin o = {nullptr, nullptr}) {
   if (v < kZc) return (float)-(zp[v] * zp[9] + zp[3 + v] * zp[10] + zp[6 + v] * zp[11]);
   if (v < kZg) return (float)zc[tri_full(v - kZc)];
   if (v < kGA) return fsqr((float)zc[7 * (v - kZg)]);
   if (v < kGB) return fsqr((float)ca[7 * (v - kGA)]);
   if (v < kTA) return fsqr((float)cb[7 * (v - kGB)]);
-  const double* t = (v == kTA ? pa : pb) + 9;
-  return (float)(std::fabs(t[0]) + std::fabs(t[1]) + std::fabs(t[2]));
+  const double *p = v == kTA ? pa : pb, *q = v == kTA ? o.a : o.b;
+  return (float)(std::fabs(from_origin(p[9], q, 9)) + std::fabs(from_origin(p[10], q, 10)) +
+                 std::fabs(from_origin(p[11], q, 11)));
 }
 // the premises of the bounds on one covariance: symmetric (the exact test
 // reads all of a trajectory covariance), |S_kl| <= sqrt(S_kk S_ll), inside
@@ -448,8 +476,10 @@ RPGO_HD bool between(const Item& x, int va, int ga, int ta, const Item& y, int v
 #pragma unroll
     for (int j = 0; j < 3; ++j) S.tr[3 * i + j] = lo(sub(Y.d(vY + 12 + tri(i + 3, j)), C.tr[3 * i + j]));
   }
-  // the magnitudes that were subtracted, |R| taken as all ones
-  const float lever = fadd(fadd(fabsv(t[0].h), fabsv(t[1].h)), fadd(fabsv(t[2].h), fadd(x.g(ta), y.g(tc))));
+  // the magnitudes that were subtracted, |R| taken as all ones (kLever: the
+  // error of the difference of the positions)
+  const float lever =
+      fadd(fadd(fabsv(t[0].h), fabsv(t[1].h)), ffma(kLever, fadd(x.g(ta), y.g(tc)), fabsv(t[2].h)));
   const float qt = ffma(lever, qr, fadd(gt, ht));
   float L[15], W[15], iD[6], h[6];
   bool ok = factor(S, L, W, iD, h) && known;
@@ -476,9 +506,10 @@ struct NoSync {
   RPGO_HD void operator()() const {}
 };
 
-// covariance and magnitudes of a composition: S <- Ad S Ad^T + Z, p <- |Ad| p + g
+// covariance and magnitudes of a composition: S <- Ad S Ad^T + Z, p <- |Ad| p + g;
+// dt: what the translation's own error adds to its magnitude
 RPGO_HD void compose_cov(const float* R, const float* t, Cov<float>& S, float (&p)[6], const float* zrr,
-                         const float* ztr, const float* ztt, const float* g) {
+                         const float* ztr, const float* ztt, const float* g, float dt) {
   Cov<float> C;
   congruence(R, t, S, C);
 #pragma unroll
@@ -499,7 +530,7 @@ RPGO_HD void compose_cov(const float* R, const float* t, Cov<float>& S, float (&
   for (int i = 0; i < 3; ++i) {
     const int a = (i + 1) % 3, b = (i + 2) % 3;
     p[i] = fadd(w[i], g[i]);
-    p[3 + i] = fadd(ffma(fabsv(t[a]), w[b], ffma(fabsv(t[b]), w[a], v[i])), g[3 + i]);
+    p[3 + i] = fadd(ffma(fadd(fabsv(t[a]), dt), w[b], ffma(fadd(fabsv(t[b]), dt), w[a], v[i])), g[3 + i]);
   }
 }
 RPGO_HD void compose_cov_z(const Item& z, Cov<float>& S, float (&p)[6]) {
@@ -520,7 +551,7 @@ RPGO_HD void compose_cov_z(const Item& z, Cov<float>& S, float (&p)[6]) {
     g[i] = z.g(kZg + i);
     g[3 + i] = z.g(kZg + 3 + i);
   }
-  compose_cov(R, t, S, p, rr, tr, tt, g);
+  compose_cov(R, t, S, p, rr, tr, tt, g, 0.f);
 }
 
 // log map of a pose in FP32 with the bounds ew (each rotation entry) and et
@@ -670,7 +701,8 @@ RPGO_HD int verdict(const Group& g, int i, int j, bool flip, float th2, Sync syn
         for (int b = 0; b < 3; ++b) R[3 * a + b] = P.R[3 * b + a].h;
         t[a] = ti[a].h;
       }
-      compose_cov(R, t, S, p, SB.rr, SB.tr, SB.tt, sb);
+      compose_cov(R, t, S, p, SB.rr, SB.tr, SB.tt, sb,
+                  fmulf(kLeverFp32, fadd(I.g(kTB1), J.g(jb ? kTB1 : kTA))));
     }
   }
   Pose L;
@@ -732,23 +764,24 @@ RPGO_HD int tri_full2(int e) {
   return 3 * i + e;
 }
 RPGO_HD D2 pack_pair2(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                      const double* zp) {
-  if (v < kCov2) return split(pa[v]);
+                      const double* zp, Origin o = {nullptr, nullptr}) {
+  if (v < kCov2) return split(v < 2 ? pa[v] : from_origin(pa[v], o.a, v));
   if (v < kPoseB2) return split(ca[tri_full2(v - kCov2)]);
-  if (v < kPoseB2 + kCov2) return split(pb[v - kPoseB2]);
+  if (v < kPoseB2 + kCov2)
+    return split(v < kPoseB2 + 2 ? pb[v - kPoseB2] : from_origin(pb[v - kPoseB2], o.b, v - kPoseB2));
   if (v < kPoseZ2) return split(cb[tri_full2(v - kPoseB2 - kCov2)]);
   return split(zp[v - kPoseZ2]);
 }
 RPGO_HD float pack_float2(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                          const double* zp, const double* zc) {
+                          const double* zp, const double* zc, Origin o = {nullptr, nullptr}) {
   if (v == 0) return (float)-(zp[0] * zp[2] + zp[1] * zp[3]);
   if (v == 1) return (float)-(zp[0] * zp[3] - zp[1] * zp[2]);
   if (v < kZg2) return (float)zc[tri_full2(v - kZc2)];
   if (v < kGA2) return fsqr((float)zc[4 * (v - kZg2)]);
   if (v < kGB2) return fsqr((float)ca[4 * (v - kGA2)]);
   if (v < kTA2) return fsqr((float)cb[4 * (v - kGB2)]);
-  const double* t = (v == kTA2 ? pa : pb) + 2;
-  return (float)(std::fabs(t[0]) + std::fabs(t[1]));
+  const double *p = v == kTA2 ? pa : pb, *q = v == kTA2 ? o.a : o.b;
+  return (float)(std::fabs(from_origin(p[2], q, 2)) + std::fabs(from_origin(p[3], q, 3)));
 }
 RPGO_HD bool cov_premise2(const double* c, bool whole) {
   bool ok = true;
@@ -838,8 +871,8 @@ RPGO_HD bool between_cov2(const Item& x, int va, int ga, int ta, const Item& y, 
   pose = between2(A, B);
   const float gv = fadd(x.g(ga), x.g(ga + 1)), hv = fadd(y.g(gc), y.g(gc + 1));
   const float qw = fadd(x.g(ga + 2), y.g(gc + 2));
-  const float lever =
-      fadd(fadd(fabsv(pose.x.h), fabsv(pose.y.h)), fadd(fadd(x.g(ta), y.g(tc)), fadd(x.g(ta), y.g(tc))));
+  // (kLever: the error of the difference of the positions)
+  const float lever = ffma(kLever, fadd(x.g(ta), y.g(tc)), fadd(fabsv(pose.x.h), fabsv(pose.y.h)));
   const float qv = ffma(lever, qw, fadd(gv, hv));
   // Ad of the inverse: rotation (c, -s), r = (y', -x') of the inverse's
   // translation; first for the main formula's first pivot, cov(v_x, v_x)
@@ -884,14 +917,14 @@ RPGO_HD bool between_cov2(const Item& x, int va, int ga, int ta, const Item& y, 
 }
 
 RPGO_HD void compose_cov2(float c, float sn, float r0, float r1, float (&S)[6], float (&p)[3], const float* Z,
-                          const float* g) {
+                          const float* g, float dt) {
   float C[6];
   congruence2(c, sn, r0, r1, S, C);
 #pragma unroll
   for (int e = 0; e < 6; ++e) S[e] = fadd(C[e], Z[e]);
   const float ac = fabsv(c), as = fabsv(sn), v0 = p[0], v1 = p[1];
-  p[0] = fadd(ffma(fabsv(r0), p[2], ffma(as, v1, fmulf(ac, v0))), g[0]);
-  p[1] = fadd(ffma(fabsv(r1), p[2], ffma(ac, v1, fmulf(as, v0))), g[1]);
+  p[0] = fadd(ffma(fadd(fabsv(r0), dt), p[2], ffma(as, v1, fmulf(ac, v0))), g[0]);
+  p[1] = fadd(ffma(fadd(fabsv(r1), dt), p[2], ffma(ac, v1, fmulf(as, v0))), g[1]);
   p[2] = fadd(p[2], g[2]);
 }
 
@@ -924,13 +957,14 @@ RPGO_HD int verdict2(const Group& g, int i, int j, bool flip, float th2, Sync sy
         for (int a = 0; a < 6; ++a) zc[a] = z.g(kZc2 + a);
 #pragma unroll
         for (int a = 0; a < 3; ++a) zg[a] = z.g(kZg2 + a);
-        compose_cov2(Z.c.h, -Z.s.h, z.g(kZt2 + 1), -z.g(kZt2), S, p, zc, zg);
+        compose_cov2(Z.c.h, -Z.s.h, z.g(kZt2 + 1), -z.g(kZt2), S, p, zc, zg, 0.f);
         if (k) Q = T;
         else P = inverse2(T);
       }
     } else {
       const Pose2D ib = inverse2(P);  // loop = Q o B
-      compose_cov2(ib.c.h, ib.s.h, ib.y.h, -ib.x.h, S, p, SB, sb);
+      compose_cov2(ib.c.h, ib.s.h, ib.y.h, -ib.x.h, S, p, SB, sb,
+                   fmulf(kLeverFp32, fadd(I.g(kTB2), J.g(jb ? kTB2 : kTA2))));
     }
   }
   const Pose2D T = compose2(Q, P);
@@ -976,18 +1010,22 @@ RPGO_HD int verdict2(const Group& g, int i, int j, bool flip, float th2, Sync sy
 }
 
 // ------------------------------------------------------------------ both
+// closure k's origins in a group: a0, b0 are the poses of closure 0's endpoints
+RPGO_HD Origin origin(const double* a0, const double* b0, bool flipped) {
+  return flipped ? Origin{b0, a0} : Origin{a0, b0};
+}
 template <int DIM>
 struct Filter;
 template <>
 struct Filter<3> {
   static constexpr int pairs = kPairs, floats = kFloats;
   RPGO_HD static D2 pair(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                         const double* z) {
-    return pack_pair(v, pa, ca, pb, cb, z);
+                         const double* z, Origin o = {nullptr, nullptr}) {
+    return pack_pair(v, pa, ca, pb, cb, z, o);
   }
   RPGO_HD static float single(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                              const double* z, const double* c) {
-    return pack_float(v, pa, ca, pb, cb, z, c);
+                              const double* z, const double* c, Origin o = {nullptr, nullptr}) {
+    return pack_float(v, pa, ca, pb, cb, z, c, o);
   }
   RPGO_HD static bool premise(const double* pa, const double* ca, const double* pb, const double* cb,
                               const double* z, const double* c) {
@@ -1003,12 +1041,12 @@ template <>
 struct Filter<2> {
   static constexpr int pairs = kPairs2, floats = kFloats2;
   RPGO_HD static D2 pair(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                         const double* z) {
-    return pack_pair2(v, pa, ca, pb, cb, z);
+                         const double* z, Origin o = {nullptr, nullptr}) {
+    return pack_pair2(v, pa, ca, pb, cb, z, o);
   }
   RPGO_HD static float single(int v, const double* pa, const double* ca, const double* pb, const double* cb,
-                              const double* z, const double* c) {
-    return pack_float2(v, pa, ca, pb, cb, z, c);
+                              const double* z, const double* c, Origin o = {nullptr, nullptr}) {
+    return pack_float2(v, pa, ca, pb, cb, z, c, o);
   }
   RPGO_HD static bool premise(const double* pa, const double* ca, const double* pb, const double* cb,
                               const double* z, const double* c) {

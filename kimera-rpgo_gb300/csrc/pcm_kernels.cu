@@ -650,7 +650,8 @@ __global__ void __launch_bounds__(32 * ROWS) k_pairwise(int n, int row_begin, co
 // per-closure data of the filter: a thread per value, the last one the closure's premises
 template <int DIM>
 __global__ void k_filter_pack(int n, const int32_t* __restrict__ sa, const int32_t* __restrict__ sb,
-                              const double* __restrict__ zp, const double* __restrict__ zc, TrajView tr,
+                              const uint8_t* __restrict__ flip, const double* __restrict__ zp,
+                              const double* __restrict__ zc, TrajView tr,
                               pf::D2* __restrict__ df, float* __restrict__ f, uint8_t* __restrict__ ok) {
   using F = pf::Filter<DIM>;
   constexpr int st = Lie<DIM>::stride, dd = Lie<DIM>::d * Lie<DIM>::d;
@@ -659,10 +660,12 @@ __global__ void k_filter_pack(int n, const int32_t* __restrict__ sa, const int32
   const size_t a = sa[k], b = sb[k];
   const double *pa = tr.pose + a * st, *pb = tr.pose + b * st, *ca = tr.cov + a * dd, *cb = tr.cov + b * dd;
   const double *z = zp + (size_t)k * st, *c = zc + (size_t)k * dd;
+  const pf::Origin o =
+      pf::origin(tr.pose + (size_t)sa[0] * st, tr.pose + (size_t)sb[0] * st, flip[k] != flip[0]);
   if (v < F::pairs)
-    df[(size_t)v * n + k] = F::pair(v, pa, ca, pb, cb, z);
+    df[(size_t)v * n + k] = F::pair(v, pa, ca, pb, cb, z, o);
   else if (v < F::pairs + F::floats)
-    f[(size_t)(v - F::pairs) * n + k] = F::single(v - F::pairs, pa, ca, pb, cb, z, c);
+    f[(size_t)(v - F::pairs) * n + k] = F::single(v - F::pairs, pa, ca, pb, cb, z, c, o);
   else
     ok[k] = tr.rot[a] && tr.rot[b] && F::premise(pa, ca, pb, cb, z, c);
 }
@@ -844,7 +847,7 @@ void pair_filter(PairFilter& p, int n, int row_begin, const int32_t* sa, const i
   constexpr int FR = 12;
   const int rows = n - row_begin;
   k_filter_pack<DIM><<<dim3(div_up(n, 128), F::pairs + F::floats + 1), 128, 0, st>>>(
-      n, sa, sb, zp, zc, tr, p.df.get(), p.f.get(), p.ok.get());
+      n, sa, sb, flip, zp, zc, tr, p.df.get(), p.f.get(), p.ok.get());
   RPGO_LAUNCHED();
   const pf::Group g{p.df.get(), p.f.get(), p.ok.get(), n};
   k_pair_filter<DIM, FR><<<dim3(div_up(n, 32), div_up(rows, FR)), dim3(32, FR), 0, st>>>(
