@@ -11,8 +11,9 @@
 // on the way: which of its two formulas each `between` takes (a positive
 // definiteness test, GeometryUtils.h:143-170) and the sign of the axis of a
 // rotation by nearly pi. Where any of them is not certain, or a bound's
-// premise fails (NaN, an asymmetric or indefinite input covariance, no
-// rotation information, values near the limits of FP32), the pair is unsure.
+// premise fails (NaN, an asymmetric trajectory covariance, a correlation
+// beyond 1, no rotation information, values near the limits of FP32, a loop
+// covariance not certain to be positive definite), the pair is unsure.
 //
 // Precision. Covariances along the odometry grow with the square of the
 // distance travelled, and `between` subtracts two of them, so `between` and
@@ -23,8 +24,8 @@
 // eps p_i p_j, with p the vector of magnitudes carried through |Ad|. With the
 // final covariance C, x the loop's log map (error e_i) and any y,
 //   d^2 >= 2 y.x - y^T C y - eps (sum p_i |y_i|)^2 - 2 sum e_i |y_i|,
-// taken at C y = x, where it is close to d^2; and with C's error relative to C
-// itself, kap = eps (sum p_i sqrt(C^-1_ii))^2 < 1,
+// taken at C y = x, where it is close to d^2; both with C's error relative to C
+// itself, kap = eps (sum p_i sqrt(C^-1_ii))^2, below 1 (else unsure), and
 //   d <= (computed d + sum e_i sqrt(C^-1_ii)) / sqrt(1 - kap),
 // or, for kap <= 1/8, the lower bound's terms 1.5 times above the computed d^2.
 #pragma once
@@ -623,8 +624,13 @@ RPGO_HD int decide(float d2, float yx, float yCy, float py, float ey, float ph, 
   // from them with a margin of 1.1
   const float eps = fmulf(1.1f, fadd(eta, 64.f * kU));
   const float low = fsub(fsub(fmulf(2.f, yx), yCy), ffma(eps, fmulf(py, py), fmulf(2.2f, ey)));
-  if (low > fmulf(th2, 1.f + 16.f * kU)) return 0;
+  // kap < 1: whatever is within eps of the computed C is positive definite,
+  // which every bound here is for. The measurements' covariances are not known
+  // to be (their premise looks at pairs of variables only), and where the exact
+  // test's C is not, it takes an elimination whose result no bound here is for.
   const float kap = fmulf(eps, fmulf(ph, ph));
+  if (!(kap < 1.f)) return 2;
+  if (low > fmulf(th2, 1.f + 16.f * kU)) return 0;
   const float d = fadd(fmulf(fsqr(d2), 1.f + 64.f * kU), fmulf(1.1f, eh));
   const float top = fmulf(th2, 1.f - 16.f * kU);
   if (kap < 0.9f && fmulf(d, d) < fmulf(top, fsub(1.f, kap))) return 1;

@@ -41,3 +41,11 @@ void pair_filter(int dim, int n, const int32_t* sa, const int32_t* sb, const uin
   else run<2>(n, sa, sb, flip, zp, zc, tp, tc, rot, th, out);
 }
 }
+
+extern "C" {
+
+// the verdict from the sums of a pair (pcm_filter.cuh, decide)
+int pair_decide(float d2, float yx, float yCy, float py, float ey, float ph, float eh, float eta, float th2) {
+  return rpgo::pf::decide(d2, yx, yCy, py, ey, ph, eh, eta, th2);
+}
+}

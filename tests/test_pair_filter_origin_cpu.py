@@ -92,3 +92,25 @@ def test_without_a_finite_origin(lib, make):
     g = make(400, 90, 30, 7)
     g["pose"][g["sb"][0], -1] = 1e300
     assert check(lib, g, 5.0) < 0.1
+
+
+def test_no_verdict_on_a_covariance_that_may_be_indefinite(lib):
+    """Far beyond the threshold, with a relative error of the covariance (here
+    1.1 * 64 * 2^-24 * ph^2) on both sides of 1."""
+    f = [C.c_float(x) for x in (100.0, 100.0, 100.0, 0.0, 0.0)]
+    rest = [C.c_float(x) for x in (0.0, 0.0, 1.0)]
+    assert lib.pair_decide(*f, C.c_float(480.0), *rest) == 0  # 0.97
+    assert lib.pair_decide(*f, C.c_float(500.0), *rest) == 2  # 1.05
+    assert lib.pair_decide(*f, C.c_float(float("nan")), *rest) == 2
+
+
+@pytest.mark.parametrize("make", [group, group2])
+def test_indefinite_closure_covariances(lib, make):
+    g = make(700, 140, 60, 11)
+    d = g["zc"].shape[1]
+    for k in range(0, len(g["sa"]), 2):
+        s = np.sqrt(np.diag(g["zc"][k])) * 10.0 ** (k % 5)
+        g["zc"][k] = np.outer(s, s) * (-0.95 + 0.05 * (k % 3))
+        g["zc"][k][np.diag_indices(d)] = s * s
+    for th in (0.01, 0.5, 5.0, 100.0):
+        check(lib, g, th)
