@@ -3,16 +3,19 @@
 //  K0 trajectory scan   Pcm::updateOdom (Pcm.h:516-557): the odometry chain
 //                       T_k = T_{k-1} o Delta_k with the covariance
 //                       Ad(Delta^-1) S Ad(Delta^-1)^T + S_Delta, sequential in
-//                       factor order (one warp; lanes split each 6x6 update).
+//                       factor order (one warp per block of the covariance).
 //  K1 odometry check    Pcm::isOdomConsistent / checkOdomConsistent
 //                       (Pcm.h:564-629), one thread per loop closure.
 //  K2 pairwise check    Pcm::areLoopsConsistent / checkLoopConsistent /
 //                       incrementAdjMatrix (Pcm.h:638-768): one thread per
 //                       closure pair (i < j), 32 consecutive i per warp, the
 //                       verdicts packed into 32-bit adjacency words with one
-//                       warp ballot; a second kernel mirrors the lower
+//                       warp ballot; a last kernel mirrors the lower
 //                       triangle into the upper one with warp bit transposes.
-// All arithmetic is the exact FP64 sequence of pcm_math.cuh.
+// All arithmetic is the exact FP64 sequence of pcm_math.cuh, but for groups of
+// 65,536 pairs of uncertain poses and more: there an FP32 test with a bound on
+// its error decides the pairs that it can (pcm_filter.cuh), and the exact
+// sequence the others, so that every verdict is the exact one.
 #include <algorithm>
 #include <type_traits>
 
@@ -633,7 +636,9 @@ __global__ void __launch_bounds__(32 * ROWS) k_pairwise(int n, int row_begin, co
 }
 
 // The PoseWithCovariance test of many pairs: FP32 with an error bound
-// decides about 99 % of them (pcm_filter.cuh), the exact FP64 test the rest.
+// decides more than 99 % of them (pcm_filter.cuh; on the walks of 2,000 and
+// 12,000 poses 99.92 and 99.5 %, wherever the map lies in its frame), the exact
+// FP64 test the rest.
 // The FP64 pipe issues a warp instruction in 64 cycles, FP32 in one, and a
 // `between` in pairs of FP32 costs about 12 FP32 instructions per FP64 FMA:
 // 10,400 instructions per 32 pairs where the exact test takes 165,000 cycles.
@@ -826,6 +831,9 @@ void launch_odom_check(int dim, int mode, int64_t count, const int32_t* si, cons
 }
 
 namespace {
+// The filter's memory, held for the call: 801 bytes per closure in 3D, 269 in
+// 2D, and the unsure pairs, a bit each, as many words as the new rows of the
+// adjacency (50 MB at 20,000 closures, 1.25 GB at 100,000).
 struct PairFilter {
   DeviceBuffer<pf::D2> df;
   DeviceBuffer<float> f;
