@@ -34,8 +34,9 @@
 // pivot (the factors keep the reciprocal of each pivot on their diagonal and
 // every solve multiplies by it). Work items spread one per SM where a level is
 // narrow, and the column work of narrow levels is split over two warps.
-// Every sum runs in an order fixed by the plan, so results do not depend on
-// scheduling. A non-positive (or NaN) pivot sets the status flag; the factor
+// Every sum runs in an order fixed by the plan and the number of CTAs (which
+// decides the levels whose backward sums are one chain per column instead of a
+// chain per lane group), so results do not depend on scheduling. A non-positive (or NaN) pivot sets the status flag; the factor
 // continues with pivot 1 so that every phase still ends, and the host treats
 // the solve as failed (as GTSAM's IndeterminantLinearSystemException).
 #include <cooperative_groups.h>
@@ -84,6 +85,7 @@ struct CholArgs {
   // ran out)
   int df_level, df_cols, df_pre_n, df_tail, df_tail_blk;
   size_t df_prod_n;
+  int df_polls;  // a wait for a word gives up after this many polls
   const int32_t *df_col, *df_blk, *df_dst, *df_pre, *df_row, *df_trow;
   double *prod, *ys, *xs;
   int32_t *df_stall, *ticket;
@@ -1041,7 +1043,7 @@ __device__ void tail_backward_item(const CholArgs& a, double* yt, int k, TileSme
 // form (chunk by chunk), so the factor has the same bits.
 // Columns are taken in level order by CTAs that are all resident
 // (cooperative launch), so the lowest unfinished column never waits for one
-// that has no CTA. Every wait for a word is bounded: after kDfSpins polls a CTA
+// that has no CTA. Every wait for a word is bounded: after df_polls polls a CTA
 // raises df_stall, on which all of them end, and the host reports the solve as
 // failed. The waits at named barriers have no limit of their own; they end
 // because every warp of the CTA comes to each of them, in an order that does
@@ -1056,7 +1058,7 @@ __device__ void tail_backward_item(const CholArgs& a, double* yt, int k, TileSme
 // 397 -> 208, 20,000 617 -> 402, 50,000 1,017 -> 780 (and 73 and 57 us for the
 // first two in the order by level of chol_plan.cpp).
 constexpr unsigned long long kEmpty = 0x7ffcd5c3a19b42e7ull;  // a NaN that no operation produces
-constexpr int kDfSpins = 1 << 21;
+constexpr int kDfSpins = 1 << 21;  // (a second or two; the longest wait is a part of one solve)
 constexpr int kPivotBar = 3;           // named barriers 3 .. 3 + D - 1: a column of L_jj is in place
 constexpr int kDfMat = kThreads - 32;  // warps 0-6: the column's blocks; warp 7: its right-hand side
 
@@ -1074,8 +1076,8 @@ __device__ __forceinline__ bool is_empty(double v) {
 // one more poll of a wait found nothing; true (in all lanes of the warp) when
 // the wait has to end
 __device__ __forceinline__ bool df_give_up(const CholArgs& a, int& spins) {
-  if ((++spins & 1023) != 0) return false;
-  if (spins >= kDfSpins) atomicExch(a.df_stall, 1);
+  if (++spins < a.df_polls && (spins & 1023) != 0) return false;
+  if (spins >= a.df_polls) atomicExch(a.df_stall, 1);
   return __any_sync(kFull, *(volatile int32_t*)a.df_stall != 0);
 }
 // Words p[0], p[step], ... (n <= N of them, 0 in lanes without) as soon as
@@ -2054,7 +2056,7 @@ int chol_grid(const SolverDev& s) {
 // poses 822 / 797 / 780 / 775 (and 513 and 845 at 20 columns per CTA); batches
 // on 76 CTAs each, 16 graphs of 200 to 2,000 poses: 124 (2) / 121 (4) / 122
 // (8) / 130 (16) ms; on 19 CTAs each: 144 (8) / 157 (16) / 197 ms (32).
-int chol_dataflow_cols(const SolverDev& s) { return 4 * chol_grid(s); }
+int chol_dataflow_cols(const SolverDev& s) { return s.df_cols >= 0 ? s.df_cols : 4 * chol_grid(s); }
 
 // kernel arguments of one solve (one system; the joint batch adds its own)
 static CholArgs make_args(SolverDev& s, CholDev& c, double lambda) {
@@ -2079,6 +2081,7 @@ static CholArgs make_args(SolverDev& s, CholDev& c, double lambda) {
   a.df_cols = (int)(p.df_col.size() / kDfColInts);
   a.df_pre_n = (int)(p.df_pre.size() / 4);
   a.df_prod_n = (size_t)p.df_products;
+  a.df_polls = s.df_polls > 0 ? s.df_polls : kDfSpins;
   a.df_tail = p.df_tail;
   a.df_tail_blk = p.df_tail_blk;
   a.df_col = c.df_col.get();

@@ -50,6 +50,9 @@ struct BatchDev {
 struct SolverDev {
   int dim = 3, d = 6, stride = 12, N = 0, F = 0;
   int coop_ctas = 0;  // CTAs of the cooperative direct solve (0: one per SM)
+  // the direct solve's dataflow part: its widest level (-1: by the number of
+  // CTAs; 0: no such part), and the polls after which a wait gives up (0: kDfSpins)
+  int df_cols = -1, df_polls = 0;
   // fill-in guard: a direct plan whose factorisation exceeds the guard's
   // flops runs its first damped system with both solvers (race = 1) and
   // keeps the faster (pcg_chosen when the PCG path won)
