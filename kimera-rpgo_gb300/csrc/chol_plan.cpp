@@ -21,11 +21,18 @@ constexpr double kUsPerFlop = 5e-6;
 // Unknowns up to which a graph's elimination order goes by level (see
 // order_variables). A long trajectory's conditioning amplifies the rounding of
 // the solve, so the estimate at which the iteration stops depends on the order
-// in the last digits: over 12 graphs each of 300, 1,000 and 2,000 poses by at
-// most 5e-13, 2e-11 and 2e-11 of its norm, but at 5,000 poses by up to 5e-9
-// and at 50,000 by 1e-7. Graphs beyond the limit keep minimum degree, and with it
+// in the last digits. Two orders' estimates differ, as a share of their norm and
+// at most over 12 graphs of a size, each by LM and by GNC: 3D 300 poses 4e-13,
+// 1,000 2e-11, 1,500 2e-10, 2,048 (the limit) 4e-10; 2D 500 2e-11, 1,000 1e-10,
+// 2,000 4e-11, 3,000 9e-11, 4,096 (the limit) 2e-10; but 3D 5,000 poses 5e-9 and
+// 50,000 1e-7. Graphs beyond the limit keep minimum degree, and with it
 // the estimates they had; theirs is the smaller gain too (5,000 poses 208 -> 148
-// us per solve, 20,000 402 -> 290, where the solve is half of an update).
+// us per solve, 20,000 402 -> 290, where the solve is half of an update). A
+// session that grows past the limit changes its order there, by those 2e-10 to
+// 4e-10. Minimum degree is no candidate below it: over 11 kinds of graphs of 60
+// to 2,000 poses its plan is up to 30 times the longer, by the time model, and
+// at best 5 % (3D) or 14 % (2D, 300 poses, 8 us) the shorter, on random edges
+// without a trajectory's order.
 constexpr int kByLevelUnknowns = 12288;
 
 // Elimination game on the variable graph: eliminating u records its current
