@@ -1123,7 +1123,7 @@ struct DfSmem {
   static constexpr int dd = D * D;
   double S[(1 + kDfMaxBlocks) * dd];  // the column's blocks, then its solved blocks
   double Lj[dd];                      // L_jj (lower part, reciprocal pivots)
-  double X[kTB][kTB + 1];             // the dense tail
+  double X[kTailMax][kTailMax + 1];   // the dense tail
 };
 
 __device__ __forceinline__ void df_mat_sync() { bar_wait(1, kDfMat); }
@@ -1381,11 +1381,11 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
   }
   __syncthreads();
   if (wi == kDfMat / 32) {
-    double v = 0.0, l[kTB];
+    double v = 0.0, l[kTailMax];
 #pragma unroll
-    for (int c = 0; c < kTB; ++c) l[c] = c <= lane && lane < n ? s.X[lane][c] : 0.0;
+    for (int c = 0; c < kTailMax; ++c) l[c] = c <= lane && lane < n ? s.X[lane][c] : 0.0;
 #pragma unroll
-    for (int c = 0; c < kTB; ++c)
+    for (int c = 0; c < kTailMax; ++c)
       if (c < n) {
         if (lane == c) v = b * l[c];
         const double yc = __shfl_sync(kFull, v, c);
@@ -1393,9 +1393,9 @@ __device__ void df_tail(const CholArgs& a, DfSmem<D>& s) {
       }
     b = v;
 #pragma unroll
-    for (int c = 0; c < kTB; ++c) l[c] = c >= lane && c < n ? s.X[c][lane] : 0.0;
+    for (int c = 0; c < kTailMax; ++c) l[c] = c >= lane && c < n ? s.X[c][lane] : 0.0;
 #pragma unroll
-    for (int c = kTB - 1; c >= 0; --c)
+    for (int c = kTailMax - 1; c >= 0; --c)
       if (c < n) {
         if (lane == c) v = b * l[c];
         const double xc = __shfl_sync(kFull, v, c);

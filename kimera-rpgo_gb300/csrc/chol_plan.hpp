@@ -31,6 +31,9 @@ constexpr int tail_slots(int d) { return 8 * (32 / d); }
 constexpr bool tail_fits(int T, int d) {
   return T * (T + 1) / 2 * d * d <= 7 * 32 && T * d * (T * d + 1) / 2 <= 6 * 32;
 }
+constexpr int kTailMax = 18;  // the scalars of the largest such tail
+static_assert(tail_fits(kTailMax / 3, 3) && !tail_fits(kTailMax / 3 + 1, 3) && tail_fits(kTailMax / 6, 6) &&
+              !tail_fits(kTailMax / 6 + 1, 6));
 
 struct CholPlan {
   int N = 0;             // variables (block columns)
