@@ -7,13 +7,14 @@
 // What the exact test computes is d = |Logmap(loop)| in the metric of the
 // loop's covariance, compared with a threshold. Its operations only matter
 // through their rounding errors, so the verdict is known as soon as d, known
-// to within E, is further than E from the threshold. Two things are decided
+// to within E, is further than E from the threshold. Some things are decided
 // on the way: which of its two formulas each `between` takes (a positive
-// definiteness test, GeometryUtils.h:143-170) and the sign of the axis of a
-// rotation by nearly pi. Where any of them is not certain, or a bound's
-// premise fails (NaN, an asymmetric trajectory covariance, a correlation
-// beyond 1, no rotation information, values near the limits of FP32, a loop
-// covariance not certain to be positive definite), the pair is unsure.
+// definiteness test, GeometryUtils.h:143-170), which formula the logarithm
+// takes, and the sign of the axis of a rotation by nearly pi. Where any of them
+// is not certain, or a bound's premise fails (NaN, an asymmetric trajectory
+// covariance, a correlation beyond 1, no rotation information, values near the
+// limits of FP32, a loop covariance not certain to be positive definite), the
+// pair is unsure.
 //
 // Precision. Covariances along the odometry grow with the square of the
 // distance travelled, and `between` subtracts two of them, so `between` and
@@ -556,8 +557,16 @@ RPGO_HD void compose_cov_z(const Item& z, Cov<float>& S, float (&p)[6]) {
 }
 
 // log map of a pose in FP32 with the bounds ew (each rotation entry) and et
-// (each translation entry); false where the axis' sign or the rotation itself
-// is not certain
+// (each translation entry); false where the axis' sign, the formula that the
+// exact test takes or the rotation itself is not certain. For a matrix that is
+// not quite a rotation (a long chain of rounded ones) the formulas on the two
+// sides of the angle's line differ, and so do those of two diagonal entries as
+// large as each other (the check of the rotation sees neither a symmetric part
+// that is off nor less than 1e-6), so both sides have to come to the same one:
+// cs has an error of at most 10 kU here, a difference of diagonal entries 2 kU.
+// The bounds are 12 times what the formulas give (worst of 4e6 rotations of all
+// angles, axes along the coordinates and pairs of them: 11 kU, and 8 kU of the
+// translation's 1-norm).
 RPGO_HD bool logmap(const Pose& T, float (&xi)[6], float& ew, float& et) {
   float R[9];
 #pragma unroll
@@ -570,6 +579,7 @@ RPGO_HD bool logmap(const Pose& T, float (&xi)[6], float& ew, float& et) {
   const float th = atan2f(sn, cs);
   const float t2 = fmulf(th, th);
   float w0, w1, w2;
+  ok = ok && fabsv(fadd(cs, 1.6f)) > 32.f * kU;
   if (cs > -1.6f) {
     const float k = th < 0.01f ? ffma(t2, 1.f / 12.f, 0.5f) : fdvd(th, sn);
     w0 = fmulf(k, vx);
@@ -580,6 +590,7 @@ RPGO_HD bool logmap(const Pose& T, float (&xi)[6], float& ew, float& et) {
     // the largest diagonal entry's axis component first
     const float s10 = fadd(R[1], R[3]), s20 = fadd(R[2], R[6]), s21 = fadd(R[5], R[7]);
     const bool i1 = R[4] > R[0], i2 = R[8] > (i1 ? R[4] : R[0]);
+    ok = ok && fabsv(fsub(R[8], i1 ? R[4] : R[0])) > 8.f * kU && (i2 || fabsv(fsub(R[4], R[0])) > 8.f * kU);
     const float dg = i2 ? R[8] : (i1 ? R[4] : R[0]);
     const float ni = fsqr(fdvd(fsub(dg, c), omc));
     const float den = fmulf(fmulf(2.f, omc), ni);
