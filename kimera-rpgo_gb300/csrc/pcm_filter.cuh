@@ -88,8 +88,10 @@ RPGO_HD float fsqr(float a) {
 RPGO_HD float fabsv(float a) { return a < 0.f ? -a : a; }  // (NaN stays NaN)
 
 constexpr float kU = 5.9604644775390625e-8f;      // 2^-24
-constexpr float kDf = 3.637978807091713e-12f;     // 2^-38: about 2.4 times the worst case of a `between`
-                                                  // (about 420 roundings of 2^-48)
+// 2^-38: 2.4 times what about 420 roundings of 2^-48, the longest way into an
+// entry of a `between`, add up to if each is as bad as can be. Worst of 400,000
+// random ones against 64-bit significands: 0.006 of the bound.
+constexpr float kDf = 3.637978807091713e-12f;
 // A difference of two positions has an error of at most kDt (|t_a| + |t_c|)
 // (1-norms): 2^-48 of each from its pair, 2^-46 from the subtraction in pairs.
 // It moves the covariances through their lever arms: by kDt (|t_a| + |t_c|)
@@ -652,7 +654,8 @@ RPGO_HD int decide(float d2, float yx, float yCy, float py, float ey, float ph, 
 
 // The translations that the pose chain goes through (1-norms); the loop's
 // translation has at most kPoseErr of their sum as error from the chain (about
-// 40 roundings of 2^-48, and a margin of 6).
+// 40 roundings of 2^-48, and a margin of 6; worst of 400,000 random chains against
+// 64-bit significands: 0.013 of the bound).
 constexpr float kPoseErr = 9.094947017729282e-13f;  // 2^-40
 template <int D>
 RPGO_HD float chain_length(const Item& I, const Item& J, int ta, int tb, int zt) {
