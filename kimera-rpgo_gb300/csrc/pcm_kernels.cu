@@ -280,8 +280,8 @@ __global__ void k_odom_prep(int64_t count, const double* __restrict__ dpose, con
 // poses are a chain of their own on another SM.
 // Bound by the latency of a step: seven FP64 instructions (448 cycles alone,
 // about 530 with three warps on the SM's FP64 pipe) and the exchange of the
-// block between its lanes twice; 790 cycles in all. 20,000 steps: 3D 18.0 ->
-// 8.0 ms (before: two warps, 13 instructions and two block barriers a step),
+// block between its lanes twice; 812 cycles in all. 20,000 steps: 3D 17.9 ->
+// 7.85 ms (before: two warps, 13 instructions and two block barriers a step),
 // 2D 20.5 -> 6.5 ms (one warp).
 constexpr int kScanChunk = 16;  // steps per chunk
 
@@ -641,13 +641,13 @@ __global__ void __launch_bounds__(32 * ROWS) k_pairwise(int n, int row_begin, co
 // FP64 test the rest.
 // The FP64 pipe issues a warp instruction in 64 cycles, FP32 in one, and a
 // `between` in pairs of FP32 costs about 12 FP32 instructions per FP64 FMA:
-// 10,400 instructions per 32 pairs where the exact test takes 165,000 cycles.
-// 3D, 4,001 closures: 35.0 -> 4.0 ms; 16,000: 556 -> 60 ms. 2D, 3,000 closures:
-// 5.3 -> 0.96 ms; 12,000: 80.7 -> 10.9 ms. Bound by FP32 issue
-// (about 0.6 of its rate); the rest is instruction fetch: the code is larger
-// than the first-level instruction cache, so the phases' loops are rolled (115
-// -> 63 ms) and the 12 warps of a block go through the phases together (-> 60
-// ms; with 4, 8 and 16 warps 64, 66 and 72 ms).
+// 10,900 instructions per 32 pairs where the exact test takes 165,000 cycles.
+// 3D, 4,001 closures: 35.0 -> 3.6 ms; 16,000: 556 -> 55 ms. 2D, 3,000 closures:
+// 5.3 -> 0.6 ms; 12,000: 80.7 -> 7.7 ms. Bound by FP32 issue (0.67 of its
+// slots). The code is larger than the first-level instruction cache, so the
+// phases' loops are rolled (16,000 closures in 3D, when the exact test still
+// took 6 ms more of it: 115 -> 63 ms) and the 12 warps of a block go through the
+// phases together (-> 60 ms; with 4, 8 and 16 warps 64, 66 and 72 ms).
 // k_pair_filter leaves its verdicts in `lower` and its unsure pairs as bits in
 // `unsure` (both one word per 32 x 1 tile); k_pair_exact gathers those bits
 // into full warps and adds the consistent ones to `lower`.
