@@ -36,9 +36,10 @@
 // narrow, and the column work of narrow levels is split over two warps.
 // Every sum runs in an order fixed by the plan and the number of CTAs (which
 // decides the levels whose backward sums are one chain per column instead of a
-// chain per lane group), so results do not depend on scheduling. A non-positive (or NaN) pivot sets the status flag; the factor
-// continues with pivot 1 so that every phase still ends, and the host treats
-// the solve as failed (as GTSAM's IndeterminantLinearSystemException).
+// chain per lane group), so results do not depend on scheduling. A
+// non-positive (or NaN) pivot sets the status flag; the factor continues with
+// pivot 1 so that every phase still ends, and the host treats the solve as
+// failed (as GTSAM's IndeterminantLinearSystemException).
 #include <cooperative_groups.h>
 
 #include "chol.hpp"
